@@ -1,5 +1,6 @@
-// Direct cross-correlation kernel (all source types and smearing modes), and
-// its batched form over whole (dump x channel) blocks.
+// Direct cross-correlation without smearing or Gaussian sources, the launch
+// of every direct variant (the smearing kernel is xcorr_smear.cuh's), and the
+// batched form over whole (dump x channel) blocks.
 //
 // Replaces the reference's warp-per-baseline kernel
 // (oskar/correlate/src/oskar_cross_correlate_cuda.cu:45-224) with a
@@ -10,10 +11,8 @@
 // correlated, then a shared-to-shared transform forms the "left" factor J B
 // (or I J in scalar mode) and the "right" factor J once per station-source
 // for the whole CTA, so the per source-baseline work is the 8 complex MACs
-// of (J_p B) J_q^H. Smearing arguments are per-station source phases
-// (phi_p - phi_q), which turns the reference's three multiply-adds per
-// source-baseline into one subtraction. FP64 mode accumulates in FP64; FP32
-// mode sums each chunk in FP32 and the chunk sums in FP64.
+// of (J_p B) J_q^H. FP64 mode accumulates in FP64; FP32 mode sums each chunk
+// in FP32 and the chunk sums in FP64.
 //
 // Work items. A launch covers items (dump t, channel c, station tile, source
 // slice); each CTA loops over items. The single-call entry points are one
@@ -29,64 +28,13 @@
 
 #include <mutex>
 
-#include "common.cuh"
+#include "xcorr_common.cuh"
+#include "xcorr_smear.cuh"
 
 namespace oskb {
 namespace {
 
-constexpr int kTile = 32;      // stations per block edge
-constexpr int kChunk = 8;      // sources per shared-memory chunk
 constexpr int kThreads = 256;  // 16 x 16 threads, 2 x 2 baselines each
-
-template <typename T>
-struct XcorrParams
-{
-    int num_src, num_st, offset_out;
-    int src_stride;  // sources per station row of jones (= num_src)
-    const T* jones;  // J [station][source], or E when K is fused
-    const T *I, *Q, *U, *V, *l, *m, *n, *a, *b, *c;
-    // Station (u, v, w) metres of dump t at st_u + t * uvw_time_stride
-    // (v and w follow at +num_st and +2 num_st in block mode).
-    const T *st_u, *st_v, *st_w, *st_x, *st_y;
-    long long uvw_time_stride;
-    double uv_min, uv_max;  // wavelengths (single call) or metres (block)
-    int uv_filter_in_metres;
-    double inv_wavelength;            // single call
-    const double* inv_wavelength_c;   // block: [channel]
-    double bw_scale;  // pi * frac_bandwidth * inv_wavelength (= pi bw / c0)
-    double ts_base;   // pi * omega_earth * time_int_sec (x inv_wavelength)
-    double gha0;                      // single call
-    const double* gha0_t;             // block: [dump]
-    double s_dec, c_dec;
-    T* vis;
-    // Items: num_times x num_channels x tiles x slices, in that nesting
-    // (slices fastest). Source slice y covers [y * slice_len,
-    // (y + 1) * slice_len). With more than one slice (single call only),
-    // each CTA writes its sums to partial[y][baseline][comp] and
-    // reduce_partials adds them to vis in slice order (deterministic).
-    int num_times, num_channels, tiles, slices, slice_len;
-    int tile_major;  // item order: tile outermost instead of innermost
-    double* partial;
-    // Fused Jones K (block mode): J = K E, K = exp(i 2 pi / lambda (u l +
-    // v m + w (n - 1))), zero where I is outside (filter_min, filter_max].
-    long long e_time_stride;  // E of dump t at jones + t * e_time_stride
-    double filter_min, filter_max;
-    // Brightness per channel (block mode): I, Q, U, V of channel c at
-    // + c * flux_channel_stride (0: the same for every channel).
-    long long flux_channel_stride;
-};
-
-template <typename T, bool MATRIX>
-struct Staging
-{
-    // Bytes of one Jones element and the cp.async copy size used for it.
-    static constexpr int ELEM = (int) sizeof(T) * (MATRIX ? 8 : 2);
-    static constexpr int COPY = ELEM >= 16 ? 16 : ELEM;
-    static constexpr int PIECES = ELEM / COPY;
-};
-
-// Per-source arrays staged with each chunk.
-enum SrcArr { kI = 0, kQ, kU, kV, kL, kM, kN, kGa, kGb, kGc, kNumSrcArr };
 
 template <typename T, bool MATRIX>
 struct Smem
@@ -103,143 +51,15 @@ struct Smem
     // row (p) and column (q) blocks.
     T2 row[NCOMP][kChunk][kTile];
     T2 col[NCOMP][kChunk][kTile];
-    // Per-station smearing phases phi and their sin, cos:
-    // [block][phi, sin, cos][source][station], bandwidth (ph) and time (ps).
-    T ph[2][3][kChunk][kTile];
-    T ps[2][3][kChunk][kTile];
-    T ga[kChunk], gb[kChunk], gc[kChunk];
-    // Per-station terms, loaded once per item: u, v, w (bandwidth phase and
-    // fused K) and the rotated x, y pair (time smearing).
+    // Station u, v, w of the fused K, loaded once per item.
     T st_uvw[2][kTile][3];
-    double st_xy[2][kTile][2];
 };
-
-// Per-item constants.
-struct ItemCtx
-{
-    int t, c, p0, q0, src_begin, src_end;
-    double inv_wavelength, ts_scale, s_ha, c_ha;
-};
-
-__device__ __forceinline__ void cp_async(void* smem, const void* gmem,
-        bool in_range, int bytes)
-{
-    const unsigned s = (unsigned) __cvta_generic_to_shared(smem);
-    const int src = in_range ? bytes : 0;  // 0: zero-fill, nothing read
-    if (bytes == 16)
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n"
-                :: "r"(s), "l"(gmem), "r"(src) : "memory");
-    else if (bytes == 8)
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n"
-                :: "r"(s), "l"(gmem), "r"(src) : "memory");
-    else
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n"
-                :: "r"(s), "l"(gmem), "r"(src) : "memory");
-}
-
-__device__ __forceinline__ void cp_async_commit()
-{
-    asm volatile("cp.async.commit_group;\n" ::: "memory");
-}
-
-__device__ __forceinline__ void cp_async_wait_all()
-{
-    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-}
-
-// Waits until at most N of this thread's cp.async groups are pending.
-template <int N>
-__device__ __forceinline__ void cp_async_wait_group()
-{
-    asm volatile("cp.async.wait_group %0;\n" :: "n"(N) : "memory");
-}
-
-// sinc(phi_p - phi_q) = sin(phi_p - phi_q) / (phi_p - phi_q), the
-// reference's smearing factor (define_cross_correlate.h:16-32), from the
-// per-station sin and cos: sin(a - b) = sin a cos b - cos a sin b. Where the
-// difference d is small the identity loses relative accuracy (its absolute
-// error is a few ulp of 1), so below |d| = tau the Taylor series of sinc is
-// summed instead, 1 - d^2/6 + d^4/120 - d^6/5040 + d^8/362880, whose
-// truncation error d^10/39916800 is below 1e-20 (FP64, tau = 0.05) and
-// 3e-11 (FP32, tau = 0.5); above tau the identity's relative error is below
-// ~1e-14 (FP64) and ~1e-6 (FP32).
-template <typename T>
-__device__ __forceinline__ T sinc_series(T d)
-{
-    const T d2 = d * d;
-    return (T) 1 + d2 * ((T) (-1.0 / 6) + d2 * ((T) (1.0 / 120) +
-            d2 * ((T) (-1.0 / 5040) + d2 * (T) (1.0 / 362880))));
-}
-
-// 1 / d for |d| >= 0.05 (FP64): the hardware's reciprocal approximation
-// refined by two steps of Newton's method for 1 / d, y' = y + y (1 - d y),
-// each of which squares the relative error (from ~2^-23 to below 2^-52,
-// then rounding). A short dependent chain instead of the IEEE division's;
-// the quotient is within an ulp or two of the correctly rounded one.
-__device__ __forceinline__ double recip_newton(double d)
-{
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
-    double e = fma(-d, y, 1.0);
-    y = fma(y, e, y);
-    e = fma(-d, y, 1.0);
-    return fma(y, e, y);
-}
-
-template <typename T>
-__device__ __forceinline__ T sinc_diff(T pa, T sa, T ca, T pb, T sb, T cb)
-{
-    const T d = pa - pb;
-    const T tau = sizeof(T) == 8 ? (T) 0.05 : (T) 0.5;
-    if constexpr (sizeof(T) == 8)
-    {
-        // both forms, then a select: no divergence between the lanes of a
-        // warp whose baselines fall on either side of tau
-        const bool small = fabs(d) < tau;
-        const T by_identity = (sa * cb - ca * sb) *
-                recip_newton(small ? (T) 1 : d);
-        const T by_series = sinc_series(d);
-        return small ? by_series : by_identity;
-    }
-    else
-    {
-        if (fabs(d) < tau) return sinc_series(d);
-        return (sa * cb - ca * sb) / d;
-    }
-}
-
-// The same factor as a numerator and a denominator (sin d, d), or
-// (series, 1) below tau, so that the bandwidth and time factors of one
-// source-baseline share a single division: used in FP32, where it is
-// faster (in FP64 the two divisions measured faster than the shared one).
-template <typename T>
-__device__ __forceinline__ void sinc_parts(T pa, T sa, T ca, T pb, T sb,
-        T cb, T& num, T& den)
-{
-    const T d = pa - pb;
-    const T tau = sizeof(T) == 8 ? (T) 0.05 : (T) 0.5;
-    // both forms, then a select (no divergence within a warp)
-    const bool small = fabs(d) < tau;
-    const T by_series = sinc_series(d);
-    num = small ? by_series : sa * cb - ca * sb;
-    den = small ? (T) 1 : d;
-}
-
-// Maps a linear block index to (bp, bq) with bp >= bq.
-__device__ __forceinline__ void tri_block(int k, int& bp, int& bq)
-{
-    int p = (int) ((sqrt(8.0 * k + 1.0) - 1.0) * 0.5);
-    while ((p + 1) * (p + 2) / 2 <= k) ++p;
-    while (p * (p + 1) / 2 > k) --p;
-    bp = p;
-    bq = k - p * (p + 1) / 2;
-}
 
 // Issues the cp.async copies of one chunk (sources [s0, min(s0 + kChunk,
 // src_end))) of both station blocks and of the per-source arrays; entries
 // outside the stations or sources are zero-filled without a global read.
 // jsrc: the Jones (or, fused, E) array of this item; NULL for identity E.
-template <typename T, bool MATRIX, bool GAUSS, bool LMN>
+template <typename T, bool MATRIX, bool LMN>
 __device__ __forceinline__ void issue_chunk(Smem<T, MATRIX>& sm,
         const XcorrParams<T>& prm, const T* jsrc, const ItemCtx& it_ctx,
         int s0)
@@ -275,12 +95,11 @@ __device__ __forceinline__ void issue_chunk(Smem<T, MATRIX>& sm,
     {
         const int k = it / kChunk, sl = it % kChunk;
         const bool want = (k == kI) || (MATRIX && k <= kV) ||
-                (LMN && k >= kL && k <= kN) || (GAUSS && k >= kGa);
+                (LMN && k >= kL && k <= kN);
         if (!want) continue;
         const T* arr = k == kI ? prm.I : k == kQ ? prm.Q : k == kU ? prm.U :
                 k == kV ? prm.V : k == kL ? prm.l : k == kM ? prm.m :
-                k == kN ? prm.n : k == kGa ? prm.a : k == kGb ? prm.b :
-                prm.c;
+                prm.n;
         const int s = s0 + sl;
         const bool in = s < src_end;
         const long long off = k <= kV ? it_ctx.c * prm.flux_channel_stride :
@@ -291,23 +110,18 @@ __device__ __forceinline__ void issue_chunk(Smem<T, MATRIX>& sm,
     cp_async_commit();
 }
 
-template <typename T, bool MATRIX, bool GAUSS, bool BW, bool TS, bool CASA,
-        bool FUSED>
-__global__ void __launch_bounds__(kThreads,
-        (sizeof(T) == 8 && !FUSED && (MATRIX ? !(GAUSS || BW || TS) : !GAUSS))
-        ? 2 : 1)
+template <typename T, bool MATRIX, bool CASA, bool FUSED>
+__global__ void __launch_bounds__(kThreads, (sizeof(T) == 8 && !FUSED) ? 2 : 1)
 xcorr_direct_kernel(const XcorrParams<T> prm)
 {
     typedef typename vec2<T>::type T2;
     typedef Smem<T, MATRIX> S;
     typedef Staging<T, MATRIX> G;
     constexpr int NC = S::NCOMP;
-    constexpr bool LMN = BW || TS || FUSED;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     S& sm = *reinterpret_cast<S*>(smem_raw);
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
     const int N = prm.num_st;
-    const long long nbl = (long long) N * (N - 1) / 2;
     const int num_items = prm.num_times * prm.num_channels * prm.tiles *
             prm.slices;
 
@@ -315,38 +129,7 @@ xcorr_direct_kernel(const XcorrParams<T> prm)
     {
     // ---- item: (dump, channel, station tile, source slice)
     ItemCtx ctx;
-    int r = item;
-    const int slice = r % prm.slices; r /= prm.slices;
-    int tile;
-    if (prm.tile_major)
-    {
-        // Consecutive items share a station tile (its E rows stay in L2).
-        const int tc = r % (prm.num_times * prm.num_channels);
-        tile = r / (prm.num_times * prm.num_channels);
-        ctx.c = tc % prm.num_channels;
-        ctx.t = tc / prm.num_channels;
-    }
-    else
-    {
-        tile = r % prm.tiles;
-        r /= prm.tiles;
-        ctx.c = r % prm.num_channels;
-        ctx.t = r / prm.num_channels;
-    }
-    {
-        int bp, bq;
-        tri_block(tile, bp, bq);
-        ctx.p0 = bp * kTile;
-        ctx.q0 = bq * kTile;
-    }
-    ctx.src_begin = slice * prm.slice_len;
-    ctx.src_end = min(prm.num_src, ctx.src_begin + prm.slice_len);
-    ctx.inv_wavelength = prm.inv_wavelength_c ?
-            prm.inv_wavelength_c[ctx.c] : prm.inv_wavelength;
-    ctx.ts_scale = prm.ts_base * ctx.inv_wavelength;
-    ctx.s_ha = ctx.c_ha = 0;
-    if (TS) sincos(prm.gha0_t ? prm.gha0_t[ctx.t] : prm.gha0, &ctx.s_ha,
-            &ctx.c_ha);
+    const int slice = decode_item(prm, item, false, ctx);
     const T* su = prm.st_u + ctx.t * prm.uvw_time_stride;
     const T* sv = prm.st_v + ctx.t * prm.uvw_time_stride;
     const T* sw = prm.st_w + ctx.t * prm.uvw_time_stride;
@@ -362,56 +145,38 @@ xcorr_direct_kernel(const XcorrParams<T> prm)
     // First chunk in flight while the per-station and baseline terms are
     // set up.
     if (ctx.src_begin < ctx.src_end)
-        issue_chunk<T, MATRIX, GAUSS, LMN>(sm, prm, jsrc, ctx,
-                ctx.src_begin);
+        issue_chunk<T, MATRIX, FUSED>(sm, prm, jsrc, ctx, ctx.src_begin);
 
-    if (LMN)
+    if (FUSED)
     {
         for (int it = tid; it < 2 * kTile; it += kThreads)
         {
             const int blk = it / kTile, stl = it % kTile;
             const int st = (blk ? ctx.q0 : ctx.p0) + stl;
             T* u = sm.st_uvw[blk][stl];
-            double* xy = sm.st_xy[blk][stl];
             u[0] = u[1] = u[2] = 0;
-            xy[0] = xy[1] = 0;
-            if (st < N)
-            {
-                u[0] = su[st]; u[1] = sv[st]; u[2] = sw[st];
-                if (TS)
-                {
-                    const double x = prm.st_x[st], y = prm.st_y[st];
-                    xy[0] = x * ctx.c_ha - y * ctx.s_ha;
-                    xy[1] = x * ctx.s_ha + y * ctx.c_ha;
-                }
-            }
+            if (st < N) { u[0] = su[st]; u[1] = sv[st]; u[2] = sw[st]; }
         }
     }
 
-    // Per-thread baseline terms.
+    // Baselines that exist and pass the uv filter, as the reference forms
+    // their lengths (oskar/correlate/define_correlate_utils.h:5-13).
     bool valid[2][2];
-    T uu2[2][2], vv2[2][2], uuvv[2][2];
 #pragma unroll
     for (int i = 0; i < 2; ++i)
 #pragma unroll
         for (int j = 0; j < 2; ++j)
         {
-            // Baseline terms as the reference forms them
-            // (oskar/correlate/define_correlate_utils.h:5-13).
             const int p = ctx.p0 + ty + 16 * i, q = ctx.q0 + tx + 16 * j;
             bool ok = (p < N) && (q < p);
-            T uu = 0, vv = 0;
             if (ok)
             {
-                uu = (su[p] - su[q]) * (T) ctx.inv_wavelength;
-                vv = (sv[p] - sv[q]) * (T) ctx.inv_wavelength;
+                const T uu = (su[p] - su[q]) * (T) ctx.inv_wavelength;
+                const T vv = (sv[p] - sv[q]) * (T) ctx.inv_wavelength;
                 const T len = sqrt(uu * uu + vv * vv);
                 ok = !(len < uv_lo || len > uv_hi);
             }
             valid[i][j] = ok;
-            uu2[i][j] = uu * uu;
-            vv2[i][j] = vv * vv;
-            uuvv[i][j] = 2 * uu * vv;
         }
 
     // Accumulators: FP64 always; FP32 mode adds per-chunk FP32 partials.
@@ -529,57 +294,12 @@ xcorr_direct_kernel(const XcorrParams<T> prm)
                 }
                 dst[0][sl][stl] = J;
             }
-            if (BW || TS)
-            {
-                // Per-station source phases (phi_p - phi_q is the
-                // reference's baseline argument), in FP64.
-                const T* u = sm.st_uvw[blk][stl];
-                const double* xy = sm.st_xy[blk][stl];
-                const double l = sm.raw_src[kL][sl], m = sm.raw_src[kM][sl];
-                const double n1 = (double) sm.raw_src[kN][sl] - 1.0;
-                T ph = 0, ps = 0;
-                if (BW)
-                    ph = (T) (((double) u[0] * l + (double) u[1] * m +
-                            (double) u[2] * n1) * prm.bw_scale);
-                if (TS)
-                    ps = (T) ((xy[0] * l + xy[1] * (prm.s_dec * m -
-                            prm.c_dec * n1)) * ctx.ts_scale);
-                if (BW)
-                {
-                    T sn, cs;
-                    sincos(ph, &sn, &cs);
-                    sm.ph[blk][0][sl][stl] = ph;
-                    sm.ph[blk][1][sl][stl] = sn;
-                    sm.ph[blk][2][sl][stl] = cs;
-                }
-                if (TS)
-                {
-                    T sn, cs;
-                    sincos(ps, &sn, &cs);
-                    sm.ps[blk][0][sl][stl] = ps;
-                    sm.ps[blk][1][sl][stl] = sn;
-                    sm.ps[blk][2][sl][stl] = cs;
-                }
-            }
         }
-        int g = 0;
-        if (GAUSS && tid < kChunk)
-        {
-            sm.ga[tid] = sm.raw_src[kGa][tid];
-            sm.gb[tid] = sm.raw_src[kGb][tid];
-            sm.gc[tid] = sm.raw_src[kGc][tid];
-            g = sm.ga[tid] != (T) 0 || sm.gb[tid] != (T) 0 ||
-                    sm.gc[tid] != (T) 0;
-        }
-        // Factors ready; the raw buffer is free. A chunk of point sources
-        // (a = b = c = 0, exp(-0) = 1 exactly) skips the Gaussian factor.
-        const bool gauss_chunk = GAUSS && __syncthreads_or(g);
-        if (!GAUSS) __syncthreads();
+        __syncthreads();  // factors ready; the raw buffer is free
 
         // ---- next chunk's copies overlap this chunk's arithmetic
         if (s0 + kChunk < ctx.src_end)
-            issue_chunk<T, MATRIX, GAUSS, LMN>(sm, prm, jsrc, ctx,
-                    s0 + kChunk);
+            issue_chunk<T, MATRIX, FUSED>(sm, prm, jsrc, ctx, s0 + kChunk);
         // ---- accumulate
         for (int sl = 0; sl < ns; ++sl)
         {
@@ -592,56 +312,6 @@ xcorr_direct_kernel(const XcorrParams<T> prm)
                     R[i][k] = sm.row[k][sl][ty + 16 * i];
                     C[i][k] = sm.col[k][sl][tx + 16 * i];
                 }
-            T smear[2][2];
-#pragma unroll
-            for (int i = 0; i < 2; ++i)
-#pragma unroll
-                for (int j = 0; j < 2; ++j)
-                {
-                    T f = (T) 1;
-                    if (GAUSS && gauss_chunk)
-                        f = exp(-(sm.ga[sl] * uu2[i][j] + sm.gb[sl] * uuvv[i][j]
-                                + sm.gc[sl] * vv2[i][j]));
-                    const int pr = ty + 16 * i, qc = tx + 16 * j;
-                    if constexpr (sizeof(T) == 8)
-                    {
-                        if (BW)
-                            f *= sinc_diff<T>(sm.ph[0][0][sl][pr],
-                                    sm.ph[0][1][sl][pr], sm.ph[0][2][sl][pr],
-                                    sm.ph[1][0][sl][qc], sm.ph[1][1][sl][qc],
-                                    sm.ph[1][2][sl][qc]);
-                        if (TS)
-                            f *= sinc_diff<T>(sm.ps[0][0][sl][pr],
-                                    sm.ps[0][1][sl][pr], sm.ps[0][2][sl][pr],
-                                    sm.ps[1][0][sl][qc], sm.ps[1][1][sl][qc],
-                                    sm.ps[1][2][sl][qc]);
-                    }
-                    else if (BW || TS)
-                    {
-                        T num = (T) 1, den = (T) 1;
-                        if (BW)
-                            sinc_parts<T>(sm.ph[0][0][sl][pr],
-                                    sm.ph[0][1][sl][pr], sm.ph[0][2][sl][pr],
-                                    sm.ph[1][0][sl][qc], sm.ph[1][1][sl][qc],
-                                    sm.ph[1][2][sl][qc], num, den);
-                        if (TS)
-                        {
-                            T n2, d2;
-                            sinc_parts<T>(sm.ps[0][0][sl][pr],
-                                    sm.ps[0][1][sl][pr], sm.ps[0][2][sl][pr],
-                                    sm.ps[1][0][sl][qc], sm.ps[1][1][sl][qc],
-                                    sm.ps[1][2][sl][qc], n2, d2);
-                            num *= n2;
-                            den *= d2;
-                        }
-                        // |den| >= 0.25 here (each factor's d is 1 or
-                        // at least tau = 0.5), well inside the range where
-                        // the fast division is accurate to 2 ulp
-                        f *= __fdividef(num, den);
-                    }
-                    smear[i][j] = f;
-                }
-            if constexpr (!(GAUSS || BW || TS))
             {
                 // No smearing: 32 FMAs per source-baseline (matrix), i.e.
                 // exactly the 64 algorithmic flops, accumulated straight
@@ -678,43 +348,6 @@ xcorr_direct_kernel(const XcorrParams<T> prm)
                             }
                         }
             }
-            else
-            {
-#pragma unroll
-            for (int i = 0; i < 2; ++i)
-#pragma unroll
-                for (int j = 0; j < 2; ++j)
-                {
-                    // L * conj-transpose(Rt): L = left factor, Rt = right.
-                    const T2* L = CASA ? C[j] : R[i];
-                    const T2* Rt = CASA ? R[i] : C[j];
-                    T* o = part[i][j];
-                    {
-                        T t[2 * NC];
-                        if constexpr (MATRIX)
-                        {
-                            // a = La Ra* + Lb Rb*, b = La Rc* + Lb Rd*,
-                            // c = Lc Ra* + Ld Rb*, d = Lc Rc* + Ld Rd*
-#define OSKB_CMAC2(OUT, X0, Y0, X1, Y1) \
-                            OUT[0] = X0.x * Y0.x + X0.y * Y0.y + X1.x * Y1.x + X1.y * Y1.y; \
-                            OUT[1] = X0.y * Y0.x - X0.x * Y0.y + X1.y * Y1.x - X1.x * Y1.y;
-                            OSKB_CMAC2((t + 0), L[0], Rt[0], L[1], Rt[1])
-                            OSKB_CMAC2((t + 2), L[0], Rt[2], L[1], Rt[3])
-                            OSKB_CMAC2((t + 4), L[2], Rt[0], L[3], Rt[1])
-                            OSKB_CMAC2((t + 6), L[2], Rt[2], L[3], Rt[3])
-#undef OSKB_CMAC2
-                        }
-                        else
-                        {
-                            t[0] = L[0].x * Rt[0].x + L[0].y * Rt[0].y;
-                            t[1] = L[0].y * Rt[0].x - L[0].x * Rt[0].y;
-                        }
-#pragma unroll
-                        for (int k = 0; k < 2 * NC; ++k)
-                            o[k] = fma(t[k], smear[i][j], o[k]);
-                    }
-                }
-            }
         }
         if (sizeof(T) == 4)
         {
@@ -740,34 +373,12 @@ xcorr_direct_kernel(const XcorrParams<T> prm)
         {
             const int p = ctx.p0 + ty + 16 * i, q = ctx.q0 + tx + 16 * j;
             if (p >= N || q >= p) continue;
-            const long long bl = baseline_index(N, p, q);
-            if (prm.partial)
-            {
-                // Every baseline of the slice is written (zero where the uv
-                // filter drops it), so the reduction reads no stale data.
-                double* out = prm.partial + (size_t) (2 * NC) * (size_t) (
-                        ((long long) slice * prm.num_times * prm.num_channels
-                        + (long long) ctx.t * prm.num_channels + ctx.c) *
-                        nbl + bl);
-#pragma unroll
-                for (int k = 0; k < 2 * NC; ++k)
-                    out[k] = !valid[i][j] ? 0.0 : (sizeof(T) == 4) ?
-                            acc[i][j][k] : (double) part[i][j][k];
-                continue;
-            }
-            if (!valid[i][j]) continue;
-            // Block layout [dump][channel][baseline] (the reference's
-            // oskar_VisBlock order, private_vis_block.h:33-57).
-            T* out = prm.vis + (size_t) (2 * NC) * (size_t) (((long long)
-                    ctx.t * prm.num_channels + ctx.c) * nbl + bl +
-                    prm.offset_out);
+            double v[2 * NC];
 #pragma unroll
             for (int k = 0; k < 2 * NC; ++k)
-            {
-                const double v = (sizeof(T) == 4) ? acc[i][j][k]
-                                                  : (double) part[i][j][k];
-                out[k] = (T) ((double) out[k] + v);
-            }
+                v[k] = (sizeof(T) == 4) ? acc[i][j][k]
+                                        : (double) part[i][j][k];
+            store_baseline<T, 2 * NC>(prm, ctx, slice, p, q, valid[i][j], v);
         }
     }  // items
 }
@@ -1048,15 +659,24 @@ reduce_partials_kernel(const double* __restrict__ partial, int num_slices,
 
 int num_sms() { return device_sm_count(); }
 
-template <typename T, bool MATRIX, bool GAUSS, bool BW, bool TS, bool CASA,
-        bool FUSED>
-void launch_one(const XcorrParams<T>& p, int grid, cudaStream_t stream)
+// Launches kernel k with its dynamic shared memory.
+template <typename T>
+void launch_kernel(void (*k)(XcorrParams<T>), size_t smem, int threads,
+        const XcorrParams<T>& p, int grid, cudaStream_t stream)
 {
-    const size_t smem = sizeof(Smem<T, MATRIX>);
-    auto k = xcorr_direct_kernel<T, MATRIX, GAUSS, BW, TS, CASA, FUSED>;
     cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
             (int) smem);
-    k<<<grid, kThreads, smem, stream>>>(p);
+    k<<<grid, threads, smem, stream>>>(p);
+}
+
+template <typename T, bool MATRIX, bool GAUSS, bool BW, bool TS, bool FUSED>
+void launch_smear(bool casa, const XcorrParams<T>& p, int grid,
+        cudaStream_t s)
+{
+    launch_kernel<T>(casa ?
+            xcorr_smear_kernel<T, MATRIX, GAUSS, BW, TS, true, FUSED> :
+            xcorr_smear_kernel<T, MATRIX, GAUSS, BW, TS, false, FUSED>,
+            sizeof(SmearSmem<T, MATRIX>), kSmearThreads, p, grid, s);
 }
 
 // Selects the kernel variant. FUSED (K formed in the staging) exists for
@@ -1065,10 +685,13 @@ template <typename T, bool MATRIX, bool FUSED>
 void launch_variant(bool casa, bool gauss, bool bw, bool ts,
         const XcorrParams<T>& p, int grid, cudaStream_t s)
 {
+    if (!gauss && !bw && !ts)
+        launch_kernel<T>(casa ? xcorr_direct_kernel<T, MATRIX, true, FUSED> :
+                xcorr_direct_kernel<T, MATRIX, false, FUSED>,
+                sizeof(Smem<T, MATRIX>), kThreads, p, grid, s);
 #define OSKB_L(G, B, S)                                                      \
-    (casa ? launch_one<T, MATRIX, G, B, S, true, FUSED>(p, grid, s)          \
-          : launch_one<T, MATRIX, G, B, S, false, FUSED>(p, grid, s))
-    if (gauss)
+    launch_smear<T, MATRIX, G, B, S, FUSED>(casa, p, grid, s)
+    else if (gauss)
     {
         if (!bw && !ts) OSKB_L(true, false, false);
         else if (bw && !ts) OSKB_L(true, true, false);
@@ -1077,8 +700,7 @@ void launch_variant(bool casa, bool gauss, bool bw, bool ts,
     }
     else
     {
-        if (!bw && !ts) OSKB_L(false, false, false);
-        else if (bw && !ts) OSKB_L(false, true, false);
+        if (bw && !ts) OSKB_L(false, true, false);
         else if (!bw && ts) OSKB_L(false, false, true);
         else OSKB_L(false, true, true);
     }
