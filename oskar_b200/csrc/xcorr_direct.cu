@@ -44,8 +44,9 @@ struct Smem
     static constexpr int NCOMP = MATRIX ? 4 : 1;
     // Raw Jones of the next chunk, landed by cp.async:
     // [block][piece][source][station] x COPY bytes, so that a warp's
-    // transform reads consecutive stations (conflict-free).
-    __align__(16) unsigned char raw[2][G::PIECES][kChunk][kTile][G::COPY];
+    // transform reads consecutive stations (conflict-free; the padding does
+    // the same for a copy's 8 sources of one station).
+    __align__(16) unsigned char raw[2][G::PIECES][kChunk][kTile + 1][G::COPY];
     T raw_src[kNumSrcArr][kChunk];
     // Factors of the current chunk: [comp][source][station] complex for the
     // row (p) and column (q) blocks.
@@ -70,18 +71,15 @@ __device__ __forceinline__ void issue_chunk(Smem<T, MATRIX>& sm,
     if (jsrc)
     {
         const unsigned char* jb = reinterpret_cast<const unsigned char*>(jsrc);
-        // Thread mapping: 8 stations x PIECES x 4 station groups x sources
-        // x blocks, so a warp reads whole elements of 8 stations and writes
-        // 8 consecutive station slots per piece.
+        // Pieces, then sources, then stations: the chunk's 8 sources of a
+        // station are contiguous, so a warp reads few rows (pages).
         constexpr int total = 2 * G::PIECES * kChunk * kTile;
         for (int it = tid; it < total; it += kThreads)
         {
-            const int a = it & 7;
-            const int pc = (it >> 3) % G::PIECES;
-            const int rest = (it >> 3) / G::PIECES;
-            const int stl = a + 8 * (rest & 3);
-            const int rest2 = rest >> 2;
-            const int sl = rest2 % kChunk, blk = rest2 / kChunk;
+            const int pc = it % G::PIECES;
+            const int rest = it / G::PIECES;
+            const int sl = rest % kChunk, rest2 = rest / kChunk;
+            const int stl = rest2 % kTile, blk = rest2 / kTile;
             const int st = (blk ? it_ctx.q0 : it_ctx.p0) + stl, s = s0 + sl;
             const bool in = st < N && s < src_end;
             const unsigned char* src = in ? jb + ((size_t) st *
@@ -389,18 +387,20 @@ xcorr_direct_kernel(const XcorrParams<T> prm)
 // Fragment-ordered operands of one chunk: per block (rows, columns),
 // kChunk / 2 k4 steps x 16 tiles of 8 rows x kFragTile doubles.
 constexpr int kFragTile = 33;
-constexpr int kFragK4 = (4 * kTile / 8) * kFragTile;
+// (+ 4: the four k4 steps a warp's transform writes at once in distinct banks)
+constexpr int kFragK4 = (4 * kTile / 8) * kFragTile + 4;
 constexpr int kFragBlock = (kChunk / 2) * kFragK4;
 
-// Shared memory of the FP64 tensor-core kernel: the raw Jones of two
-// chunks and the fragment-ordered operands of two chunks, so that one
+// Shared memory of the FP64 tensor-core kernel: the raw Jones of the next
+// chunk and the fragment-ordered operands of two chunks, so that one
 // chunk's products run while the next chunk is transformed (one barrier per
 // chunk).
 struct DmmaSmem
 {
-    // [buffer][block][piece][source][station] x 16 bytes
-    __align__(16) unsigned char raw[2][2][4][kChunk][kTile][16];
-    double src[2][kChunk][4];        // [buffer][source][I, Q, U, V]
+    // [warp][piece][element] x 16 bytes: the next chunk's Jones; a warp's 64
+    // elements are 8 stations x 8 sources
+    __align__(16) unsigned char raw[kThreads / 32][4][64][16];
+    double src[2][4][kChunk];        // [buffer][I, Q, U, V][source]
     double frag[2][2 * kFragBlock];  // [buffer][rows block, columns block]
 };
 
@@ -412,43 +412,47 @@ __device__ __forceinline__ void dmma_m8n8k4(double& d0, double& d1,
                  : "+d"(d0), "+d"(d1) : "d"(a), "d"(b));
 }
 
-// Warp w stages and transforms source sl = w of every chunk, both blocks
-// (64 elements): its copies land 8 stations x 4 pieces per instruction
-// (whole 64-byte elements of 8 stations, coalesced; 4 x 128 contiguous
-// bytes in shared memory), and its own cp.async wait plus __syncwarp make
-// them visible to its lanes, so no block barrier is needed before the
-// transform. Lanes 0-3 stage the source's I, Q, U, V.
-__device__ __forceinline__ void dmma_issue(DmmaSmem& sm, int buf,
+// Warp w stages and transforms stations 8 (w % 4) .. + 7 of block w / 4 for
+// every chunk: the 8 sources of a station are 512 contiguous bytes, one copy
+// instruction, and the warp's own cp.async wait plus __syncwarp make them
+// visible to its lanes, so no block barrier is needed before the transform.
+__device__ __forceinline__ void dmma_issue(DmmaSmem& sm,
         const XcorrParams<double>& prm, const ItemCtx& ctx, int s0)
 {
-    const int lane = threadIdx.x & 31, sl = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const unsigned char* jb = reinterpret_cast<const unsigned char*>(
             prm.jones);
-    const int s = s0 + sl;
+    const int st0 = (warp >= 4 ? ctx.q0 : ctx.p0) + 8 * (warp & 3);
+    const int pc = lane & 3, s = s0 + (lane >> 2);
     const bool src_in = s < ctx.src_end;
-    const int a = lane & 7, pc = lane >> 3;
 #pragma unroll
     for (int i = 0; i < 8; ++i)
     {
-        const int blk = i >> 2, stl = 8 * (i & 3) + a;
-        const int st = (blk ? ctx.q0 : ctx.p0) + stl;
+        const int st = st0 + i;
         const bool in = st < prm.num_st && src_in;
         const unsigned char* src = in ? jb + ((size_t) st * prm.src_stride +
                 s) * 64 + 16 * pc : jb;
-        cp_async(sm.raw[buf][blk][pc][sl][stl], src, in, 16);
-    }
-    if (lane < 4)
-    {
-        const double* arr = lane == 0 ? prm.I : lane == 1 ? prm.Q :
-                lane == 2 ? prm.U : prm.V;
-        cp_async(&sm.src[buf][sl][lane], src_in ? arr + s : prm.I, src_in,
-                8);
+        cp_async(sm.raw[warp][pc][8 * i + (lane >> 2)], src, in, 16);
     }
     cp_async_commit();
 }
 
-// Left factor J B (rows unless CASA) and right factor J of lane stl's two
-// elements of the warp's source, written in fragment order: W entry (row
+// I, Q, U, V of one chunk's sources, by one warp, into buffer b.
+constexpr int kSrcWarpDmma = 7;   // (one that transforms after its products)
+
+__device__ __forceinline__ void dmma_issue_src(DmmaSmem& sm,
+        const XcorrParams<double>& prm, const ItemCtx& ctx, int s0, int b)
+{
+    const int lane = threadIdx.x & 31, k = lane >> 3, sl = lane & 7;
+    const double* arr = k == 0 ? prm.I : k == 1 ? prm.Q : k == 2 ? prm.U :
+            prm.V;
+    const bool in = s0 + sl < ctx.src_end;
+    cp_async(&sm.src[b][k][sl], in ? arr + s0 + sl : prm.I, in, 8);
+    cp_async_commit();
+}
+
+// Left factor J B (rows unless CASA) and right factor J of each lane's two
+// elements of the chunk, written in fragment order: W entry (row
 // r, k) of a block at frag[k / 4][r / 8][4 (r % 8) + k % 4] (tiles of 8 rows
 // padded to kFragTile doubles against bank conflicts), so the mma.sync
 // operand of lane (g, t) = (r % 8, k % 4) is one 8-byte load per lane (row
@@ -458,20 +462,23 @@ __device__ __forceinline__ void dmma_transform(DmmaSmem& sm, int buf,
         int fbuf)
 {
     typedef double2 T2;
-    const int stl = threadIdx.x & 31, sl = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int blk = warp >> 2;
     __syncwarp();  // the warp's own copies, landed, visible to all lanes
 #pragma unroll
-    for (int blk = 0; blk < 2; ++blk)
+    for (int half = 0; half < 2; ++half)
     {
+        const int el = lane + 32 * half;
+        const int stl = 8 * (warp & 3) + (el >> 3), sl = el & 7;
         Mat2<double> J;
-        J.a = *reinterpret_cast<const T2*>(sm.raw[buf][blk][0][sl][stl]);
-        J.b = *reinterpret_cast<const T2*>(sm.raw[buf][blk][1][sl][stl]);
-        J.c = *reinterpret_cast<const T2*>(sm.raw[buf][blk][2][sl][stl]);
-        J.d = *reinterpret_cast<const T2*>(sm.raw[buf][blk][3][sl][stl]);
+        J.a = *reinterpret_cast<const T2*>(sm.raw[warp][0][el]);
+        J.b = *reinterpret_cast<const T2*>(sm.raw[warp][1][el]);
+        J.c = *reinterpret_cast<const T2*>(sm.raw[warp][2][el]);
+        J.d = *reinterpret_cast<const T2*>(sm.raw[warp][3][el]);
         if ((blk == 0) != CASA)
         {
-            const double I = sm.src[buf][sl][0], Q = sm.src[buf][sl][1];
-            const T2 buv = T2{sm.src[buf][sl][2], sm.src[buf][sl][3]};
+            const double I = sm.src[buf][0][sl], Q = sm.src[buf][1][sl];
+            const T2 buv = T2{sm.src[buf][2][sl], sm.src[buf][3][sl]};
             const T2 buvc = T2{buv.x, -buv.y};
             const double xx = I + Q, yy = I - Q;
             Mat2<double> M;
@@ -507,9 +514,8 @@ __device__ __forceinline__ void dmma_transform(DmmaSmem& sm, int buf,
 // The 128 x 128 G tile is split over 8 warps as 4 (rows) x 2 (columns) warp
 // tiles of 32 x 64 = 4 x 8 m8n8 accumulators; a k4 step is two sources.
 // Accumulation is FP64 throughout (no brightness factorisation, so any B).
-// Pipeline per chunk c: copies of chunk c + 2 in flight, products of chunk
-// c on the tensor pipe, transform of chunk c + 1 on the FP64 pipe, one
-// barrier.
+// Pipeline per chunk c: products of chunk c on the tensor pipe, transform of
+// chunk c + 1 on the FP64 pipe, copies of chunk c + 2 in flight, one barrier.
 template <bool CASA>
 __global__ void __launch_bounds__(kThreads, 1)
 xcorr_dmma_kernel(const XcorrParams<double> prm)
@@ -546,56 +552,80 @@ xcorr_dmma_kernel(const XcorrParams<double> prm)
 #pragma unroll
         for (int ns = 0; ns < 8; ++ns) acc[ms][ns][0] = acc[ms][ns][1] = 0.0;
 
+    // Transform of chunk c into fragment buffer c & 1, then the copies of
+    // chunk c + 1 into the warp's raw buffer. The per-source values of chunk
+    // c, in buffer c & 1, are copied an iteration earlier by one warp, whose
+    // own transform of that iteration (after its products) waits for them.
+    const auto advance = [&](int c)
+    {
+        cp_async_wait_all();
+        dmma_transform<CASA>(sm, c & 1, c & 1);
+        __syncwarp();
+        if (c + 1 < nchunks)
+            dmma_issue(sm, prm, ctx, ctx.src_begin + (c + 1) * kChunk);
+    };
+    const auto issue_src = [&](int c)
+    {
+        if (warp == kSrcWarpDmma && c < nchunks)
+            dmma_issue_src(sm, prm, ctx, ctx.src_begin + c * kChunk, c & 1);
+    };
+    // Each scheduler runs warps w and w + 4: the first transforms the next
+    // chunk and issues its copies before its products of this one, the
+    // second after, so that one's transform and copies (1,100 and 1,300 cycles
+    // of a chunk) run under the other's products (2,048). With all warps in
+    // step the tensor pipe was idle meanwhile: 128 stations x 12,000 sources
+    // (K, join and this kernel) 560 us, 419 with the split and with the
+    // slices of choose_slices.
+    const bool early = warp < kThreads / 64;
+    // a warp whose 8 x 16 stations hold no baseline (above the diagonal,
+    // past the last station) skips the products
+    const bool active = ctx.p0 + 8 * wm < N && ctx.q0 + 16 * wn < N &&
+            ctx.p0 + 8 * wm + 7 > ctx.q0 + 16 * wn;
+
     __syncthreads();  // the previous item is done with shared memory
     if (nchunks > 0)
     {
-        dmma_issue(sm, 0, prm, ctx, ctx.src_begin);
-        if (nchunks > 1)
-        {
-            dmma_issue(sm, 1, prm, ctx, ctx.src_begin + kChunk);
-            cp_async_wait_group<1>();
-        }
-        else
-        {
-            cp_async_wait_group<0>();
-        }
-        dmma_transform<CASA>(sm, 0, 0);
+        issue_src(0);
+        dmma_issue(sm, prm, ctx, ctx.src_begin);
+        cp_async_wait_all();
+        __syncthreads();   // chunk 0's source values are there
+        issue_src(1);
+        advance(0);
         __syncthreads();
     }
     for (int c = 0; c < nchunks; ++c)
     {
-        const int s0 = ctx.src_begin + c * kChunk;
-        // copies of chunk c + 2 into the raw buffer chunk c used (this
-        // warp transformed its own elements of it already)
-        if (c + 2 < nchunks)
-            dmma_issue(sm, c & 1, prm, ctx, s0 + 2 * kChunk);
-        // ---- products of chunk c: 4 k4 steps of 2 sources
-        const double* fbase = sm.frag[c & 1];
-#pragma unroll
-        for (int k4 = 0; k4 < kChunk / 2; ++k4)
+        issue_src(c + 2);
+#pragma unroll 1
+        for (int step = 0; step < 2; ++step)
         {
-            const double* fa = fbase + k4 * kFragK4;
-            const double* fb = fa + kFragBlock;
-            double a[4], b[8];
+            if ((step == 0) == early)
+            {
+                if (c + 1 < nchunks) advance(c + 1);
+                continue;
+            }
+            if (!active) continue;
+            // ---- products of chunk c: 4 k4 steps of 2 sources
+            const double* fbase = sm.frag[c & 1];
 #pragma unroll
-            for (int ms = 0; ms < 4; ++ms)
-                a[ms] = fa[(4 * wm + ms) * kFragTile + lane];
+            for (int k4 = 0; k4 < kChunk / 2; ++k4)
+            {
+                const double* fa = fbase + k4 * kFragK4;
+                const double* fb = fa + kFragBlock;
+                double a[4], b[8];
 #pragma unroll
-            for (int ns = 0; ns < 8; ++ns)
-                b[ns] = fb[(8 * wn + ns) * kFragTile + lane];
-#pragma unroll
-            for (int ms = 0; ms < 4; ++ms)
+                for (int ms = 0; ms < 4; ++ms)
+                    a[ms] = fa[(4 * wm + ms) * kFragTile + lane];
 #pragma unroll
                 for (int ns = 0; ns < 8; ++ns)
-                    dmma_m8n8k4(acc[ms][ns][0], acc[ms][ns][1], a[ms],
-                            b[ns]);
-        }
-        // ---- transform of chunk c + 1 while the products run
-        if (c + 1 < nchunks)
-        {
-            if (c + 2 < nchunks) cp_async_wait_group<1>();
-            else cp_async_wait_group<0>();
-            dmma_transform<CASA>(sm, (c + 1) & 1, (c + 1) & 1);
+                    b[ns] = fb[(8 * wn + ns) * kFragTile + lane];
+#pragma unroll
+                for (int ms = 0; ms < 4; ++ms)
+#pragma unroll
+                    for (int ns = 0; ns < 8; ++ns)
+                        dmma_m8n8k4(acc[ms][ns][0], acc[ms][ns][1], a[ms],
+                                b[ns]);
+            }
         }
         __syncthreads();
     }
@@ -750,6 +780,50 @@ int tiles_for(int num_st)
     return nb * (nb + 1) / 2;
 }
 
+// Number of source slices for `items` tiles of `chunks` source chunks each on
+// `slots` resident CTAs: the one that minimises the waves of CTAs times the
+// chunks of a slice plus a fixed cost per slice, about two chunks' time
+// (filling the pipeline, and writing and reducing its partial sums of `bytes`
+// bytes). Few long slices that fill the slots once beat many short ones
+// where the tiles take equal time: 128 stations (10 tiles) x 12,000 sources
+// in 14 slices instead of 119. Tiles with dead patches take less (work: the
+// sum in whole tiles), and then more slices than slots even out: the
+// estimate is half a slice beyond the average.
+int choose_slices(long long items, double work, int chunks, int slots,
+        size_t bytes)
+{
+    constexpr int kFixed = 2;
+    constexpr size_t kMostBytes = (size_t) 512 << 20;
+    const int most = (int) min((long long) chunks, (8LL * slots + items - 1)
+            / items);
+    int best = 1;
+    double best_cost = 0;
+    for (int s = 1; s <= most && (s == 1 || s * bytes <= kMostBytes); ++s)
+    {
+        const int len = (chunks + s - 1) / s;
+        if ((chunks + len - 1) / len != s) continue;
+        const long long waves = (items * s + slots - 1) / slots;
+        const double even = work < (double) items ? max(1.0, work * s / slots
+                + 0.5) : (double) waves;
+        const double cost = (waves > 1 ? min(even, (double) waves) : 1.0) *
+                len + (s > 1 ? (double) (waves * kFixed) : 0.0);
+        if (s == 1 || cost < best_cost)
+        {
+            best = s;
+            best_cost = cost;
+        }
+    }
+    return best;
+}
+
+// Work of a smearing launch's tiles, in whole tiles: the share of the 8 x 8
+// patches that hold a baseline.
+double smear_tiles(int num_st)
+{
+    const double n = (num_st + 7) / 8;
+    return n * (n + 1) / 2 / 16;
+}
+
 // One call: one dump, one channel, sources split into slices.
 template <typename T, bool MATRIX>
 int xcorr_dispatch(bool casa, bool gauss, XcorrParams<T> p,
@@ -762,11 +836,17 @@ int xcorr_dispatch(bool casa, bool gauss, XcorrParams<T> p,
     if ((uintptr_t) p.jones % Staging<T, MATRIX>::COPY != 0)
         return OSKB_ERR_INVALID_ARGUMENT;
     const int tiles = tiles_for(p.num_st);
-    // Split the sources into slices so that about four waves of two CTAs
-    // per SM are in flight, each slice at least 64 sources long.
-    const int max_slices = (p.num_src + 8 * kChunk - 1) / (8 * kChunk);
-    int slices = (8 * num_sms() + tiles - 1) / tiles;
-    slices = max(1, min(slices, max_slices));
+    // CTAs that run at a time: one per SM for the tensor-pipe and smearing
+    // kernels, two for the register-tiled one in FP64
+    const bool dmma = use_dmma<T, MATRIX>(gauss, bw, ts);
+    const int per_sm = sizeof(T) == 8 && !dmma && !gauss && !bw && !ts ? 2 :
+            1;
+    const int chunks = (p.num_src + kChunk - 1) / kChunk;
+    const size_t slice_bytes = (size_t) p.num_st * (p.num_st - 1) / 2 *
+            (MATRIX ? 8 : 2) * sizeof(double);
+    int slices = choose_slices(tiles, gauss || bw || ts ?
+            smear_tiles(p.num_st) : (double) tiles, chunks,
+            per_sm * num_sms(), slice_bytes);
     if (const char* e = getenv("OSKB_XCORR_SLICES")) slices = max(1, atoi(e));
     int slice_len = (p.num_src + slices - 1) / slices;
     slice_len = (slice_len + kChunk - 1) / kChunk * kChunk;
@@ -791,7 +871,7 @@ int xcorr_dispatch(bool casa, bool gauss, XcorrParams<T> p,
             p.slice_len = p.num_src;
         }
     }
-    if (use_dmma<T, MATRIX>(gauss, bw, ts))
+    if (dmma)
         launch_dmma(casa, p, tiles * slices, stream);
     else
         launch_variant<T, MATRIX, false>(casa, gauss, bw, ts, p,
@@ -939,15 +1019,15 @@ int block_dispatch(bool casa, bool gauss, bool bw, bool ts, XcorrParams<T> p,
     if (tc_items > 0x7fffffffLL) return OSKB_ERR_INVALID_ARGUMENT;
     const BlockSchedule s = block_schedule<T>(casa, gauss, bw, ts, p, stream);
     p.tile_major = s.tile_major;
-    // Too few (dump, channel, tile) items to fill the GPU: split the
-    // sources too (at least 64 per slice), the slices' sums reduced into
-    // vis in slice order afterwards.
-    const long long want = 4LL * num_sms();
-    if (tc_items < want)
+    // Few (dump, channel, tile) items: split the sources too, the slices'
+    // sums reduced into vis in slice order afterwards.
+    if (tc_items < 4LL * num_sms())
     {
-        const int max_slices = (p.num_src + 8 * kChunk - 1) / (8 * kChunk);
-        int slices = (int) min((long long) max_slices,
-                (want + tc_items - 1) / tc_items);
+        const long long tc = (long long) p.num_times * p.num_channels;
+        int slices = choose_slices(tc_items, gauss || bw || ts ?
+                tc * smear_tiles(p.num_st) : (double) tc_items,
+                (p.num_src + kChunk - 1) / kChunk, num_sms(), (size_t) tc *
+                p.num_st * (p.num_st - 1) / 2 * 8 * sizeof(double));
         if (slices > 1)
         {
             int len = (p.num_src + slices - 1) / slices;
