@@ -21,6 +21,7 @@
 // CTA cooperatively before the main loop, so there is no second launch.
 // In FP64 the element loops take their phase factors from a shared-memory
 // table (trig_table.cuh) instead of a library sincos per element-direction.
+#include <algorithm>
 #include <climits>
 
 #include "beam_common.cuh"
@@ -29,8 +30,18 @@
 namespace oskb {
 namespace {
 
-constexpr int kThreads = 128;
+constexpr int kThreads = 256;
 constexpr int kChunk = 512;
+constexpr int kCtasPerSm = 2;
+// directions per thread: most items, and those of the last round (FP32 works
+// on pairs)
+template <typename T>
+constexpr int dirs_big(int num_types)
+{
+    // FP64 sums of several element types leave no registers for more
+    return sizeof(T) == 4 || num_types == 1 ? 4 : num_types == 2 ? 2 : 1;
+}
+template <typename T> constexpr int kDirsSmall = sizeof(T) == 8 ? 1 : 2;
 
 struct BeamFlags
 {
@@ -38,17 +49,15 @@ struct BeamFlags
     int scalar;  // complex beam of the pattern amplitude (Stokes-I mode)
 };
 
-// e^{i ph} for the normalisation direction: ph in table steps through
-// the shared table in FP64, in radians through sincosf in FP32.
-__device__ __forceinline__ void phase_factor(const double2* table, double ph,
-        double* s, double* c)
+// Bit pattern of |v| as a float rounded up: orders as the values do, with
+// NaN above everything.
+__device__ __forceinline__ unsigned abs_bits(double v)
 {
-    trig_steps_checked(table, ph, s, c);
+    return __float_as_uint(__double2float_ru(fabs(v)));
 }
-__device__ __forceinline__ void phase_factor(const double2*, float ph,
-        float* s, float* c)
+__device__ __forceinline__ unsigned abs_bits(float v)
 {
-    sincosf(ph, s, c);
+    return __float_as_uint(fabsf(v));
 }
 
 template <typename T>
@@ -90,6 +99,28 @@ __device__ __forceinline__ void type_pattern(const TypeParams<T>& tp, int t,
             swap_xy, p);
 }
 
+// The same in one of the beam's directions; rot as element_pattern_rotated
+// (FP64; the FP32 pattern keeps the reference's angles, whose rounding near
+// the dipole's axis its single-precision results carry).
+template <typename T>
+__device__ __forceinline__ void direction_pattern(const TypeParams<T>& tp,
+        int t, T X, T Y, T Z, T dphi1, T dphi2, const T* rot, int swap_xy,
+        T p[4])
+{
+    if (tp.kind[t] == 1)
+    {
+        p[0] = p[3] = (T) 1;
+        p[1] = p[2] = (T) 0;
+        return;
+    }
+    if constexpr (sizeof(T) == 8)
+        element_pattern_rotated<T>(X, Y, Z, dphi1, dphi2, rot, tp.kL[t],
+                tp.cos_kL[t], swap_xy, p);
+    else
+        element_pattern<T>(X, Y, Z, false, dphi1, dphi2, tp.kL[t],
+                tp.cos_kL[t], swap_xy, p);
+}
+
 // Element taper of type t at polar angle theta = atan2(|(X, Y)|, Z),
 // applied after the pole normalisation (oskar_element_evaluate.c:159-174;
 // define_apply_element_taper_{cosine,gaussian}.h).
@@ -103,217 +134,355 @@ __device__ __forceinline__ T type_taper(const TypeParams<T>& tp, int t, T X,
     return exp(-(theta * theta) * tp.taper_param[t]);
 }
 
-// (ar, ai)[t] += w e^{i ph} for the element's type t only: register selects
-// over a compile-time number of types, so the accumulators stay in
-// registers. One type: the plain complex multiply-add.
-template <typename T, int NT>
-__device__ __forceinline__ void add_term(T* ar, T* ai,
-        typename vec2<T>::type w, int type, T sn, T cs)
+// Terms of one element, staged once per (station, chunk): position, gain and
+// the phase of its weight in table steps (reduced to one turn). FP32 terms
+// are stored twice, as packed pairs {v, v} for two directions at a time.
+template <typename T, bool IS3D> struct ElementTerms;
+template <bool IS3D> struct ElementTerms<double, IS3D>
 {
-    if constexpr (NT == 1)
-    {
-        ar[0] += cs * w.x - w.y * sn;
-        ai[0] += sn * w.x + w.y * cs;
-    }
-    else
-    {
+    double2 xy[kChunk], pg[kChunk];
+    double z[IS3D ? kChunk : 1];
+};
+template <bool IS3D> struct ElementTerms<float, IS3D>
+{
+    float4 xy[kChunk], pg[kChunk];
+    float2 z[IS3D ? kChunk : 1];
+};
+
+template <bool IS3D>
+__device__ __forceinline__ void put_element(ElementTerms<double, IS3D>& el,
+        int i, double x, double y, double z, double p, double g)
+{
+    el.xy[i] = make_double2(x, y);
+    el.pg[i] = make_double2(p, g);
+    if (IS3D) el.z[i] = z;
+}
+template <bool IS3D>
+__device__ __forceinline__ void put_element(ElementTerms<float, IS3D>& el,
+        int i, float x, float y, float z, float p, float g)
+{
+    el.xy[i] = make_float4(x, x, y, y);
+    el.pg[i] = make_float4(p, p, g, g);
+    if (IS3D) el.z[i] = make_float2(z, z);
+}
+
+// Phase factors e^{i u} of element i in the thread's ND directions, u in
+// table steps.
+template <bool IS3D, int ND>
+__device__ __forceinline__ void element_factors(
+        const ElementTerms<double, IS3D>& el, const double2* table, int i,
+        const double (&kX)[ND], const double (&kY)[ND],
+        const double (&kZ)[ND], double (&sn)[ND], double (&cs)[ND],
+        double& gain)
+{
+    const double2 xy = el.xy[i], pg = el.pg[i];
+    gain = pg.y;
 #pragma unroll
-        for (int t = 0; t < NT; ++t)
-        {
-            const T wx = type == t ? w.x : (T) 0;
-            const T wy = type == t ? w.y : (T) 0;
-            ar[t] += cs * wx - wy * sn;
-            ai[t] += sn * wx + wy * cs;
-        }
+    for (int j = 0; j < ND; ++j)
+    {
+        double u = fma(kY[j], xy.y, pg.x);
+        if (IS3D) u = fma(kZ[j], el.z[i], u);
+        u = fma(kX[j], xy.x, u);
+        Trig<double>::sincos(table, u, &sn[j], &cs[j]);
+    }
+}
+template <bool IS3D, int ND>
+__device__ __forceinline__ void element_factors(
+        const ElementTerms<float, IS3D>& el, const float2* table, int i,
+        const float (&kX)[ND], const float (&kY)[ND], const float (&kZ)[ND],
+        float (&sn)[ND], float (&cs)[ND], float& gain)
+{
+    const ulonglong2 xy = *reinterpret_cast<const ulonglong2*>(&el.xy[i]);
+    const ulonglong2 pg = *reinterpret_cast<const ulonglong2*>(&el.pg[i]);
+    float g2;
+    unpack2(pg.y, gain, g2);
+#pragma unroll
+    for (int j = 0; j < ND; j += 2)
+    {
+        f32x2 u = fma2(pack2(kY[j], kY[j + 1]), xy.y, pg.x);
+        if (IS3D)
+            u = fma2(pack2(kZ[j], kZ[j + 1]),
+                    *reinterpret_cast<const f32x2*>(&el.z[i]), u);
+        u = fma2(pack2(kX[j], kX[j + 1]), xy.x, u);
+        Trig<float>::sincos2(table, u, &sn[j], &cs[j]);
+    }
+}
+
+// The same through the library, for phases the table does not cover.
+template <typename T, bool IS3D, int ND>
+__device__ __forceinline__ void element_factors_exact(
+        const ElementTerms<T, IS3D>& el, int i, const T (&kX)[ND],
+        const T (&kY)[ND], const T (&kZ)[ND], T (&sn)[ND], T (&cs)[ND],
+        T& gain)
+{
+    T x, y, p;
+    if constexpr (sizeof(T) == 8) { x = el.xy[i].x; y = el.xy[i].y; }
+    else { x = el.xy[i].x; y = el.xy[i].z; }
+    if constexpr (sizeof(T) == 8) { p = el.pg[i].x; gain = el.pg[i].y; }
+    else { p = el.pg[i].x; gain = el.pg[i].z; }
+    T z = 0;
+    if constexpr (IS3D && sizeof(T) == 8) z = el.z[i];
+    if constexpr (IS3D && sizeof(T) == 4) z = el.z[i].x;
+#pragma unroll
+    for (int j = 0; j < ND; ++j)
+    {
+        T u = fma(kY[j], y, p);
+        if (IS3D) u = fma(kZ[j], z, u);
+        u = fma(kX[j], x, u);
+        Trig<T>::exact(u, &sn[j], &cs[j]);
+    }
+}
+
+// (ar, ai)[t] += gain e^{i u} for the element's type t only: register
+// selects over a compile-time number of types, so the accumulators stay in
+// registers.
+template <typename T, int NT>
+__device__ __forceinline__ void add_term(T* ar, T* ai, T gain, int type,
+        T sn, T cs)
+{
+#pragma unroll
+    for (int t = 0; t < NT; ++t)
+    {
+        const T g = (NT == 1 || type == t) ? gain : (T) 0;
+        ar[t] = fma(g, cs, ar[t]);
+        ai[t] = fma(g, sn, ai[t]);
     }
 }
 
 template <typename T, bool IS3D, int NT>
-__global__ void __launch_bounds__(kThreads)
-station_beam_kernel(int num_elements, const T* __restrict__ el_x,
-        const T* __restrict__ el_y, const T* __restrict__ el_z,
-        const T* __restrict__ meas_x, const T* __restrict__ meas_y,
-        const T* __restrict__ meas_z, const T* __restrict__ cable,
-        const T* __restrict__ weight_factors,
-        const int* __restrict__ element_type,
-        const double* __restrict__ orientation_x,
-        const double* __restrict__ orientation_y, TypeParams<T> tp,
-        BeamFlags flags, T wavenumber, const double* __restrict__ beam_enu,
-        const double* __restrict__ norm_enu, int num_dir,
-        const T* __restrict__ dir_x, const T* __restrict__ dir_y,
-        const T* __restrict__ dir_z, int directions_per_station, int rows,
-        T* __restrict__ norm_af, T* __restrict__ beam)
+struct BeamSmem
 {
+    typename Trig<T>::Entry table[Trig<T>::kSize];
+    ElementTerms<T, IS3D> el;
+    int type[NT > 1 ? kChunk : 1];
+    T red[2][NT][kThreads / 32];
+    T rot[NT][4];        // element_pattern_rotated's, of the item's station
+    unsigned bound[3];   // largest |x|, |y|, |z| of the chunk, float bits
+};
+
+// Arguments of a station-beam launch (the entry points').
+template <typename T>
+struct BeamArgs
+{
+    int num_elements;
+    const T *el_x, *el_y, *el_z, *meas_x, *meas_y, *meas_z, *cable;
+    const T* weight_factors;
+    const int* element_type;
+    const double *orientation_x, *orientation_y;
+    TypeParams<T> tp;
+    BeamFlags flags;
+    double wavenumber;
+    const double *beam_enu, *norm_enu;
+    int num_dir;
+    const T *dir_x, *dir_y, *dir_z;
+    int directions_per_station;
     // rows: 0 all four; 1 the x feed's (xx, xy); 2 the y feed's (yx, yy).
     // With one feed per launch the final normalisation needs both feeds'
     // array factors at the normalisation direction: the launch writes its
     // own to norm_af[station][type] (complex) and leaves the scaling to
     // feeds_finalise_kernel.
-    typedef typename vec2<T>::type T2;
-    __shared__ T2 s_w[kChunk];
-    __shared__ T s_x[kChunk], s_y[kChunk], s_z[IS3D ? kChunk : 1];
-    __shared__ int s_type[NT > 1 ? kChunk : 1];
-    __shared__ T s_red[2][NT][kThreads / 32];
-    // FP64: phase factors of the element loops from the shared table
-    __shared__ double2 s_trig[sizeof(T) == 8 ? kTrigTableSize : 1];
-    const int st = blockIdx.y;
-    const int d = blockIdx.x * kThreads + threadIdx.x;
-    const bool active = d < num_dir;
-    const size_t el0 = (size_t) st * num_elements;
-    const size_t dir0 = directions_per_station ? (size_t) st * num_dir : 0;
-    const int per_dir = flags.scalar ? 1 : 4;
-    T2* out = reinterpret_cast<T2*>(beam) +
-            per_dir * ((size_t) st * num_dir + d);
+    int rows;
+    T* norm_af;
+    T* beam;
+};
 
-    const T bx = (T) beam_enu[3 * st], by = (T) beam_enu[3 * st + 1],
+// Beam of station st in directions d_first + thread + j kThreads, j < ND.
+// The weight of an element, f e^{-i k (r_m . b + cable)}, is folded into the
+// element loop as a gain |f| and a phase in table steps, so an
+// element-direction is one phase (2 or 3 multiply-adds), one table phase
+// factor and one real-by-complex multiply-add: in FP64 17 operations
+// (planar) against 21 with a complex weight and the 128-entry table.
+template <typename T, bool IS3D, int NT, int ND>
+__device__ __forceinline__ void station_beam_item(BeamSmem<T, IS3D, NT>& sm,
+        const BeamArgs<T>& arg, int st, int d_first)
+{
+    typedef typename vec2<T>::type T2;
+    typedef Trig<T> Tr;
+    const int num_elements = arg.num_elements, num_dir = arg.num_dir;
+    const BeamFlags& flags = arg.flags;
+    const TypeParams<T>& tp = arg.tp;
+    const double* beam_enu = arg.beam_enu;
+    const int rows = arg.rows;
+    const int d0 = d_first + threadIdx.x;
+    const size_t el0 = (size_t) st * num_elements;
+    const size_t dir0 = arg.directions_per_station ? (size_t) st * num_dir : 0;
+    const int per_dir = flags.scalar ? 1 : 4;
+    T2* out = reinterpret_cast<T2*>(arg.beam) + per_dir * ((size_t) st * num_dir);
+
+    const double bx = (T) beam_enu[3 * st], by = (T) beam_enu[3 * st + 1],
             bz = (T) beam_enu[3 * st + 2];
     if (beam_enu[3 * st + 2] < 0.0)  // pointing below the horizon
     {
-        if (active)
-            for (int k = 0; k < per_dir; ++k) out[k] = T2{(T) 0, (T) 0};
+#pragma unroll
+        for (int j = 0; j < ND; ++j)
+        {
+            const int d = d0 + j * kThreads;
+            if (d < num_dir)
+                for (int k = 0; k < per_dir; ++k)
+                    out[(size_t) per_dir * d + k] = T2{(T) 0, (T) 0};
+        }
         return;
-    }
-    if constexpr (sizeof(T) == 8)
-    {
-        trig_table_fill(s_trig);
-        __syncthreads();
     }
     // element orientations per (station, type)
     T dphi1[NT], dphi2[NT];
 #pragma unroll
     for (int t = 0; t < NT; ++t)
     {
-        dphi1[t] = (T) (kPi / 2 - (orientation_x[st * NT + t] + kPi / 2));
-        dphi2[t] = (T) (kPi / 2 - orientation_y[st * NT + t]);
+        dphi1[t] = (T) (kPi / 2 - (arg.orientation_x[st * NT + t] + kPi / 2));
+        dphi2[t] = (T) (kPi / 2 - arg.orientation_y[st * NT + t]);
     }
 
-    T X = 0, Y = 0, Z = 0;
-    if (active)
+    T X[ND], Y[ND], Z[ND], kX[ND], kY[ND], kZ[ND];
+    const double k_steps = arg.wavenumber * Tr::kStepsPerRadian;
+#pragma unroll
+    for (int j = 0; j < ND; ++j)
     {
-        X = dir_x[dir0 + d];
-        Y = dir_y[dir0 + d];
-        Z = dir_z[dir0 + d];
+        const int d = d0 + j * kThreads;
+        X[j] = Y[j] = Z[j] = 0;
+        if (d < num_dir)
+        {
+            X[j] = arg.dir_x[dir0 + d];
+            Y[j] = arg.dir_y[dir0 + d];
+            Z[j] = arg.dir_z[dir0 + d];
+        }
+        // phase per metre in table steps, rounded once
+        kX[j] = (T) (k_steps * (double) X[j]);
+        kY[j] = (T) (k_steps * (double) Y[j]);
+        kZ[j] = (T) (k_steps * (double) Z[j]);
     }
     T nX = 0, nY = 0, nZ = 1;
     if (flags.normalise_final)
     {
-        nX = (T) norm_enu[3 * st];
-        nY = (T) norm_enu[3 * st + 1];
-        nZ = (T) norm_enu[3 * st + 2];
+        nX = (T) arg.norm_enu[3 * st];
+        nY = (T) arg.norm_enu[3 * st + 1];
+        nZ = (T) arg.norm_enu[3 * st + 2];
     }
-    // Phase factors per element coordinate: radians in FP32, table steps
-    // (radians x 64 / pi) in FP64.
-    const T to_steps = sizeof(T) == 8 ? (T) kTrigStepsPerRadian : (T) 1;
-    const T kX = wavenumber * X * to_steps, kY = wavenumber * Y * to_steps,
-            kZ = wavenumber * Z * to_steps;
-    const T knX = wavenumber * nX * to_steps, knY = wavenumber * nY * to_steps,
-            knZ = wavenumber * nZ * to_steps;
+    const T knX[1] = {(T) (k_steps * (double) nX)},
+            knY[1] = {(T) (k_steps * (double) nY)},
+            knZ[1] = {(T) (k_steps * (double) nZ)};
 
-    // array factors per element type: this thread's direction (ar, ai) and
+    // array factors per element type: the thread's directions (ar, ai) and
     // the normalisation direction (nr, ni)
-    T ar[NT], ai[NT], nr[NT], ni[NT];
+    T ar[ND][NT], ai[ND][NT], nr[NT], ni[NT];
 #pragma unroll
-    for (int t = 0; t < NT; ++t) ar[t] = ai[t] = nr[t] = ni[t] = (T) 0;
+    for (int t = 0; t < NT; ++t)
+    {
+        nr[t] = ni[t] = (T) 0;
+#pragma unroll
+        for (int j = 0; j < ND; ++j) ar[j][t] = ai[j][t] = (T) 0;
+    }
     for (int e0 = 0; e0 < num_elements; e0 += kChunk)
     {
         const int ne = min(kChunk, num_elements - e0);
+        __syncthreads();  // table filled; the previous chunk is consumed
+        if (threadIdx.x < 3) sm.bound[threadIdx.x] = 0;
+        if (e0 == 0 && threadIdx.x >= 32 && threadIdx.x < 32 + 2 * NT)
+        {
+            const int t = (threadIdx.x - 32) >> 1, f = threadIdx.x & 1;
+            T d1 = 0, s1, c1;
+#pragma unroll
+            for (int k = 0; k < NT; ++k)
+                if (k == t) d1 = f ? dphi2[k] : dphi1[k];
+            sincos(d1, &s1, &c1);
+            sm.rot[t][2 * f] = c1;
+            sm.rot[t][2 * f + 1] = s1;
+        }
+        __syncthreads();
+        unsigned ex = 0, ey = 0, ez = 0;
         for (int t = threadIdx.x; t < ne; t += kThreads)
         {
             const size_t g = el0 + e0 + t;
-            const T mx = meas_x ? meas_x[g] : el_x[g];
-            const T my = meas_y ? meas_y[g] : el_y[g];
-            const T mz = meas_z ? meas_z[g] : (el_z ? el_z[g] : (T) 0);
-            const T p = wavenumber * (mx * bx + my * by + mz * bz +
-                    (cable ? cable[g] : (T) 0));
-            T sn, cs;
-            sincos(-p, &sn, &cs);
-            if (weight_factors)
+            const T x = arg.el_x[g], y = arg.el_y[g], z = arg.el_z ? arg.el_z[g] : (T) 0;
+            const double wx = arg.meas_x ? arg.meas_x[g] : x;
+            const double wy = arg.meas_y ? arg.meas_y[g] : y;
+            const double wz = arg.meas_z ? arg.meas_z[g] : z;
+            // the weight's phase in table steps and its gain
+            double p = -k_steps * (wx * bx + wy * by + wz * bz +
+                    (arg.cable ? (double) arg.cable[g] : 0.0));
+            T gain = (T) 1;
+            if (arg.weight_factors)
             {
                 // element errors x apodisation, applied to the DFT weight
-                const T2 f = reinterpret_cast<const T2*>(weight_factors)[g];
-                const T re = cs * f.x - sn * f.y;
-                sn = cs * f.y + sn * f.x;
-                cs = re;
+                const T2 f = reinterpret_cast<const T2*>(arg.weight_factors)[g];
+                gain = hypot(f.x, f.y);
+                p += atan2((double) f.y, (double) f.x) * Tr::kStepsPerRadian;
             }
-            s_w[t] = T2{cs, sn};
+            p -= Tr::kEntries * rint(p * (1.0 / Tr::kEntries));
+            put_element(sm.el, t, x, y, z, (T) p, gain);
             int type = 0;
             if constexpr (NT > 1)
             {
-                type = element_type ? element_type[g] : 0;
-                s_type[t] = type;
+                type = arg.element_type ? arg.element_type[g] : 0;
+                sm.type[t] = type;
             }
-            s_x[t] = el_x[g];
-            s_y[t] = el_y[g];
-            if (IS3D) s_z[t] = el_z[g];
+            ex = max(ex, abs_bits(x));
+            ey = max(ey, abs_bits(y));
+            if (IS3D) ez = max(ez, abs_bits(z));
             // The normalisation direction: elements split across threads.
             if (flags.normalise_final)
             {
-                T ph = knX * s_x[t] + knY * s_y[t];
-                if (IS3D) ph += knZ * s_z[t];
+                T u = fma(knY[0], y, (T) p);
+                if (IS3D) u = fma(knZ[0], z, u);
+                u = fma(knX[0], x, u);
                 T s2, c2;
-                phase_factor(s_trig, ph, &s2, &c2);
-                add_term<T, NT>(nr, ni, T2{cs, sn}, type, s2, c2);
+                Tr::checked(sm.table, u, &s2, &c2);
+                add_term<T, NT>(nr, ni, gain, type, s2, c2);
             }
         }
-        __syncthreads();
-        if (active)
+        ex = __reduce_max_sync(0xffffffffu, ex);
+        ey = __reduce_max_sync(0xffffffffu, ey);
+        if (IS3D) ez = __reduce_max_sync(0xffffffffu, ez);
+        if ((threadIdx.x & 31) == 0)
         {
-            if constexpr (sizeof(T) == 8)
-            {
-                // Branch-free table loop; a thread that met a phase the
-                // table does not cover redoes the chunk with sincos.
-                T ar0[NT], ai0[NT];
+            atomicMax(&sm.bound[0], ex);
+            atomicMax(&sm.bound[1], ey);
+            if (IS3D) atomicMax(&sm.bound[2], ez);
+        }
+        __syncthreads();
+        if (d0 < num_dir)
+        {
+            // The table covers every phase of the chunk when the largest
+            // possible one is covered (false for NaN); otherwise the chunk
+            // goes through the library.
+            bool covered = true;
 #pragma unroll
-                for (int t = 0; t < NT; ++t)
-                {
-                    ar0[t] = ar[t];
-                    ai0[t] = ai[t];
-                }
-                bool covered = true;
+            for (int j = 0; j < ND; ++j)
+            {
+                T bound = fabs(kX[j]) * (T) __uint_as_float(sm.bound[0]) +
+                        fabs(kY[j]) * (T) __uint_as_float(sm.bound[1]) +
+                        (T) Tr::kEntries;
+                if (IS3D)
+                    bound += fabs(kZ[j]) * (T) __uint_as_float(sm.bound[2]);
+                covered &= bound < (T) Tr::kLimit;
+            }
+            T sn[ND], cs[ND], gain;
+            if (covered)
+            {
 #pragma unroll 4
                 for (int i = 0; i < ne; ++i)
                 {
-                    T ph = kX * s_x[i] + kY * s_y[i];
-                    if (IS3D) ph += kZ * s_z[i];
-                    T sn, cs;
-                    trig_steps_sincos(s_trig, ph, &sn, &cs, covered);
-                    add_term<T, NT>(ar, ai, s_w[i], NT > 1 ? s_type[i] : 0,
-                            sn, cs);
-                }
-                if (!covered)
-                {
+                    element_factors<IS3D, ND>(sm.el, sm.table, i, kX, kY, kZ,
+                            sn, cs, gain);
 #pragma unroll
-                    for (int t = 0; t < NT; ++t)
-                    {
-                        ar[t] = ar0[t];
-                        ai[t] = ai0[t];
-                    }
-                    for (int i = 0; i < ne; ++i)
-                    {
-                        T ph = kX * s_x[i] + kY * s_y[i];
-                        if (IS3D) ph += kZ * s_z[i];
-                        T sn, cs;
-                        trig_steps_exact(ph, &sn, &cs);
-                        add_term<T, NT>(ar, ai, s_w[i],
-                                NT > 1 ? s_type[i] : 0, sn, cs);
-                    }
+                    for (int j = 0; j < ND; ++j)
+                        add_term<T, NT>(ar[j], ai[j], gain,
+                                NT > 1 ? sm.type[i] : 0, sn[j], cs[j]);
                 }
             }
             else
             {
-#pragma unroll 4
+#pragma unroll 1
                 for (int i = 0; i < ne; ++i)
                 {
-                    T ph = kX * s_x[i] + kY * s_y[i];
-                    if (IS3D) ph += kZ * s_z[i];
-                    T sn, cs;
-                    sincosf(ph, &sn, &cs);
-                    add_term<T, NT>(ar, ai, s_w[i], NT > 1 ? s_type[i] : 0,
-                            sn, cs);
+                    element_factors_exact<T, IS3D, ND>(sm.el, i, kX, kY, kZ,
+                            sn, cs, gain);
+#pragma unroll
+                    for (int j = 0; j < ND; ++j)
+                        add_term<T, NT>(ar[j], ai[j], gain,
+                                NT > 1 ? sm.type[i] : 0, sn[j], cs[j]);
                 }
             }
         }
-        __syncthreads();
     }
 
     // Element normalisation: 1 / |pattern at the pole|, per type.
@@ -333,7 +502,7 @@ station_beam_kernel(int num_elements, const T* __restrict__ el_x,
     const T array_scale = flags.normalise_array ?
             (T) (1.0 / num_elements) : (T) 1;
 
-    // Final normalisation: amplitude of the beam in the normalisation
+    // Final normalisation: amplitude of the arg.beam in the normalisation
     // direction (block reduction of its array factors first).
     T final_scale = (T) 1;
     if (flags.normalise_final)
@@ -348,8 +517,8 @@ station_beam_kernel(int num_elements, const T* __restrict__ el_x,
             }
             if ((threadIdx.x & 31) == 0)
             {
-                s_red[0][t][threadIdx.x >> 5] = nr[t];
-                s_red[1][t][threadIdx.x >> 5] = ni[t];
+                sm.red[0][t][threadIdx.x >> 5] = nr[t];
+                sm.red[1][t][threadIdx.x >> 5] = ni[t];
             }
         }
         __syncthreads();
@@ -359,8 +528,8 @@ station_beam_kernel(int num_elements, const T* __restrict__ el_x,
             nr[t] = ni[t] = 0;
             for (int w = 0; w < kThreads / 32; ++w)
             {
-                nr[t] += s_red[0][t][w];
-                ni[t] += s_red[1][t][w];
+                nr[t] += sm.red[0][t][w];
+                ni[t] += sm.red[1][t][w];
             }
             // A normalisation direction below the horizon is blanked, as in
             // the reference, which then divides by zero.
@@ -368,13 +537,13 @@ station_beam_kernel(int num_elements, const T* __restrict__ el_x,
         }
         if (rows != 0)
         {
-            if (blockIdx.x == 0 && threadIdx.x == 0)
+            if (d0 == 0)
             {
 #pragma unroll
                 for (int t = 0; t < NT; ++t)
                 {
-                    norm_af[2 * ((size_t) st * NT + t)] = nr[t];
-                    norm_af[2 * ((size_t) st * NT + t) + 1] = ni[t];
+                    arg.norm_af[2 * ((size_t) st * NT + t)] = nr[t];
+                    arg.norm_af[2 * ((size_t) st * NT + t) + 1] = ni[t];
                 }
             }
         }
@@ -434,54 +603,115 @@ station_beam_kernel(int num_elements, const T* __restrict__ el_x,
             final_scale = (T) 1 / sqrt(amp / (T) 2);
         }
     }
-    if (!active) return;
+#pragma unroll 1
+    for (int j = 0; j < ND; ++j)
+    {
+        const int d = d0 + j * kThreads;
+        if (d >= num_dir) break;
+        T2* o = out + (size_t) per_dir * d;
+        T x = X[0], y = Y[0], z = Z[0], fr[NT], fi[NT];
+#pragma unroll
+        for (int t = 0; t < NT; ++t)
+        {
+            fr[t] = ar[0][t];
+            fi[t] = ai[0][t];
+        }
+#pragma unroll
+        for (int k = 1; k < ND; ++k)
+            if (j == k)
+            {
+                x = X[k];
+                y = Y[k];
+                z = Z[k];
+#pragma unroll
+                for (int t = 0; t < NT; ++t)
+                {
+                    fr[t] = ar[k][t];
+                    fi[t] = ai[k][t];
+                }
+            }
+        const bool blank = z < (T) 0;
+        if (flags.scalar)
+        {
+            // pattern amplitude sqrt(sum p_k^2 / 2)
+            // (define_evaluate_dipole_pattern.h:51-75) times the array
+            // factor
+            T2 v{(T) 0, (T) 0};
+#pragma unroll
+            for (int t = 0; t < NT; ++t)
+            {
+                T pt[4];
+                direction_pattern<T>(tp, t, x, y, z, dphi1[t], dphi2[t],
+                        sm.rot[t], flags.swap_xy, pt);
+                const T a = sqrt(half_frobenius<T>(pt, 1, 0)) *
+                        type_taper<T>(tp, t, x, y, z) * pole_scale[t];
+                v.x += a * fr[t] * array_scale;
+                v.y += a * fi[t] * array_scale;
+            }
+            if (blank) v = T2{(T) 0, (T) 0};
+            o[0] = T2{v.x * final_scale, v.y * final_scale};
+            continue;
+        }
+        T p[NT][4];
+#pragma unroll
+        for (int t = 0; t < NT; ++t)
+        {
+            direction_pattern<T>(tp, t, x, y, z, dphi1[t], dphi2[t],
+                    sm.rot[t], flags.swap_xy, p[t]);
+            const T taper = type_taper<T>(tp, t, x, y, z);
+            for (int k = 0; k < 4; ++k) p[t][k] *= taper;
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+        {
+            // The reference's order: pattern (normalised), times the
+            // weighted element sum, times the DFT norm, then the final
+            // scale.
+            T2 v{(T) 0, (T) 0};
+#pragma unroll
+            for (int t = 0; t < NT; ++t)
+            {
+                const T pk = p[t][k] * pole_scale[t];
+                v.x += pk * fr[t] * array_scale;
+                v.y += pk * fi[t] * array_scale;
+            }
+            if (blank) v = T2{(T) 0, (T) 0};
+            v.x *= final_scale;
+            v.y *= final_scale;
+            if (rows == 0 || (rows == 1) == (k < 2)) o[k] = v;
+        }
+    }
+}
 
-    const bool blank = Z < (T) 0;
-    if (flags.scalar)
+// One CTA takes items in turn, with its table filled once: first `full`
+// (station, block of kThreads x BIG directions) items in whole rounds of the
+// grid, then the rest in quarters or halves of kThreads x SMALL directions,
+// so that the last round is short: at 128 stations x 12,000 directions a
+// grid of 296 has 5.2 rounds of 1,024 directions, and a whole sixth round
+// would idle most of the chip. More directions per thread share the staged
+// element terms (FP64: 629 us with four against 668 us with one on that
+// shape, before the split).
+template <typename T, bool IS3D, int NT, int BIG, int SMALL>
+__global__ void __launch_bounds__(kThreads, kCtasPerSm)
+station_beam_kernel(const __grid_constant__ BeamArgs<T> arg, int blocks,
+        int items, int full)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    BeamSmem<T, IS3D, NT>& sm =
+            *reinterpret_cast<BeamSmem<T, IS3D, NT>*>(smem_raw);
+    Trig<T>::fill(sm.table);
+    for (int item = blockIdx.x; item < full; item += gridDim.x)
+        station_beam_item<T, IS3D, NT, BIG>(sm, arg, item / blocks,
+                item % blocks * (kThreads * BIG));
+    constexpr int PARTS = BIG / SMALL;
+    for (int part = blockIdx.x; part < (items - full) * PARTS;
+            part += gridDim.x)
     {
-        // pattern amplitude sqrt(sum p_k^2 / 2)
-        // (define_evaluate_dipole_pattern.h:51-75) times the array factor
-        T2 v{(T) 0, (T) 0};
-#pragma unroll
-        for (int t = 0; t < NT; ++t)
-        {
-            T pt[4];
-            type_pattern<T>(tp, t, X, Y, Z, false, dphi1[t], dphi2[t],
-                    flags.swap_xy, pt);
-            const T a = sqrt(half_frobenius<T>(pt, 1, 0)) *
-                    type_taper<T>(tp, t, X, Y, Z) * pole_scale[t];
-            v.x += a * ar[t] * array_scale;
-            v.y += a * ai[t] * array_scale;
-        }
-        if (blank) v = T2{(T) 0, (T) 0};
-        out[0] = T2{v.x * final_scale, v.y * final_scale};
-        return;
-    }
-    T p[NT][4];
-#pragma unroll
-    for (int t = 0; t < NT; ++t)
-    {
-        type_pattern<T>(tp, t, X, Y, Z, false, dphi1[t], dphi2[t],
-                flags.swap_xy, p[t]);
-        const T taper = type_taper<T>(tp, t, X, Y, Z);
-        for (int k = 0; k < 4; ++k) p[t][k] *= taper;
-    }
-    for (int k = 0; k < 4; ++k)
-    {
-        // The reference's order: pattern (normalised), times the weighted
-        // element sum, times the DFT norm, then the final scale.
-        T2 v{(T) 0, (T) 0};
-#pragma unroll
-        for (int t = 0; t < NT; ++t)
-        {
-            const T pk = p[t][k] * pole_scale[t];
-            v.x += pk * ar[t] * array_scale;
-            v.y += pk * ai[t] * array_scale;
-        }
-        if (blank) v = T2{(T) 0, (T) 0};
-        v.x *= final_scale;
-        v.y *= final_scale;
-        if (rows == 0 || (rows == 1) == (k < 2)) out[k] = v;
+        const int item = full + part / PARTS;
+        const int d = (item % blocks * PARTS + part % PARTS) *
+                (kThreads * SMALL);
+        if (d < arg.num_dir)
+            station_beam_item<T, IS3D, NT, SMALL>(sm, arg, item / blocks, d);
     }
 }
 
@@ -642,23 +872,41 @@ int station_beam_aa(int num_stations, int num_elements, const T* el_x,
             element_kind, taper_kind, taper_param, frequency_hz, &tp))
         return err;
     const double c0 = 299792458.0;
-    const T wavenumber = (T) (2.0 * kPi * frequency_hz / c0);
+    const double wavenumber = 2.0 * kPi * frequency_hz / c0;
     BeamFlags flags{normalise_element, normalise_array, normalise_final,
             swap_xy, scalar};
-    dim3 grid((num_directions + kThreads - 1) / kThreads, num_stations);
+    const int big = dirs_big<T>(num_element_types);
+    const int parts = big / kDirsSmall<T>;
+    const int blocks = (int) (((long long) num_directions + kThreads * big -
+            1) / (kThreads * big));
+    const long long items = (long long) blocks * num_stations;
+    if (items > INT_MAX / parts) return OSKB_ERR_INVALID_ARGUMENT;
+    const int slots = kCtasPerSm * device_sm_count();
+    const int full = (int) (items / slots * slots);
+    const int grid = full ? slots : (int) std::min<long long>(slots, items *
+            parts);
+    const BeamArgs<T> arg = {num_elements, el_x, el_y, el_z, meas_x, meas_y,
+            meas_z, cable, weight_factors, element_type, orientation_x,
+            orientation_y, tp, flags, wavenumber, beam_enu, norm_enu,
+            num_directions, x, y, z, directions_per_station, rows, norm_af,
+            beam};
     cudaStream_t s = as_stream(stream);
-#define OSKB_BEAM(D, NT) station_beam_kernel<T, D, NT><<<grid, kThreads, 0,    \
-        s>>>(num_elements, el_x, el_y, el_z, meas_x, meas_y, meas_z, cable,  \
-        weight_factors, element_type, orientation_x, orientation_y, tp,      \
-        flags, wavenumber, beam_enu, norm_enu, num_directions, x, y, z,      \
-        directions_per_station, rows, norm_af, beam)
+#define OSKB_BEAM(D, NT)                                                     \
+    {                                                                        \
+        auto k = station_beam_kernel<T, D, NT, dirs_big<T>(NT),              \
+                kDirsSmall<T>>;                                              \
+        const int smem = (int) sizeof(BeamSmem<T, D, NT>);                   \
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, \
+                smem);                                                       \
+        k<<<grid, kThreads, smem, s>>>(arg, blocks, (int) items, full);      \
+    }
 #define OSKB_BEAM_NT(D)                                                      \
     switch (num_element_types)                                               \
     {                                                                        \
-    case 1: OSKB_BEAM(D, 1); break;                                          \
-    case 2: OSKB_BEAM(D, 2); break;                                          \
-    case 3: OSKB_BEAM(D, 3); break;                                          \
-    default: OSKB_BEAM(D, 4); break;                                         \
+    case 1: OSKB_BEAM(D, 1) break;                                           \
+    case 2: OSKB_BEAM(D, 2) break;                                           \
+    case 3: OSKB_BEAM(D, 3) break;                                           \
+    default: OSKB_BEAM(D, 4) break;                                          \
     }
     if (is_3d) { OSKB_BEAM_NT(true) } else { OSKB_BEAM_NT(false) }
 #undef OSKB_BEAM_NT

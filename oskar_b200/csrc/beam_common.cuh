@@ -60,4 +60,45 @@ __device__ __forceinline__ void element_pattern(T X, T Y, T Z, bool pole,
     p[3] = swap_xy ? xp : yp;
 }
 
+// The same for a direction away from the zenith from its components alone:
+// with r = |(X, Y)| and h = |(X, Y, Z)|, the polar angle has sine r / h and
+// cosine Z / h, the azimuth cosine X / r and sine Y / r, and the elements'
+// azimuth offsets add by rotation (rot: cos dphi1, sin dphi1, cos dphi2,
+// sin dphi2, once per station). About 125 FP64 operations against 350 with
+// the inverse tangents and their sines and cosines. Directions where r
+// vanishes (the zenith, whose azimuth is that of the signed zeros) take
+// element_pattern.
+template <typename T>
+__device__ __forceinline__ void element_pattern_rotated(T X, T Y, T Z,
+        T dphi1, T dphi2, const T* rot, T kL, T cos_kL, int swap_xy, T p[4])
+{
+    const T r2 = X * X + Y * Y;
+    if (!(r2 > (sizeof(T) == 8 ? (T) 1e-280 : (T) 1e-30)))
+    {
+        element_pattern<T>(X, Y, Z, false, dphi1, dphi2, kL, cos_kL, swap_xy,
+                p);
+        return;
+    }
+    const T ri = rsqrt(r2), hi = rsqrt(r2 + Z * Z);
+    const T st = r2 * ri * hi, ct = Z * hi;
+    const T c0 = X * ri, s0 = Y * ri;
+#pragma unroll
+    for (int f = 0; f < 2; ++f)
+    {
+        const T cp = c0 * rot[2 * f] - s0 * rot[2 * f + 1];
+        const T sp = s0 * rot[2 * f] + c0 * rot[2 * f + 1];
+        const T denom = (T) 1 + cp * cp * (ct * ct - (T) 1);
+        T e_theta = (T) 0, e_phi = (T) 0;
+        if (denom != (T) 0)
+        {
+            const T t = (cos(kL * cp * st) - cos_kL) / denom;
+            e_theta = -cp * ct * t;
+            e_phi = sp * t;
+        }
+        const int o = (f == 0) == (swap_xy == 0) ? 0 : 2;
+        p[o] = e_theta;
+        p[o + 1] = e_phi;
+    }
+}
+
 }  // namespace oskb

@@ -30,7 +30,7 @@
 // three integer operations, against one library sincos.
 #pragma once
 
-#include "common.cuh"
+#include "f32x2.cuh"
 
 namespace oskb {
 
@@ -101,5 +101,140 @@ __device__ __forceinline__ void trig_steps_checked(const double2* table,
     trig_steps_sincos(table, u, s, c, covered);
     if (!covered) trig_steps_exact(u, s, c);
 }
+
+// ---------------------------------------------------------------------------
+// The station beam's larger tables, with shorter series. Entry j of copy c is
+// element kCopies j + c, as above (FP32: 16 copies of 8-byte entries, for
+// half-warp requests). N entries: h = 2 pi / N, |x| = |h f| <= pi / N.
+//   FP64, N = 512 (64 KB): sin to x^5 (the omitted x^7/7! < 7e-20) and
+//     cos - 1 to x^4 with the x^6 term economised into the lower two
+//     (Chebyshev; what is left is below 5e-18): 13 operations.
+//   FP32, N = 256 (32 KB): sin to x^3 (x^5/5! < 3e-12) and cos - 1 as one
+//     economised x^2 term (left: 2e-10): 11 operations.
+// The caller bounds the phase: |u| < kLimit, where round(u) still sits in
+// the low bits of u + 1.5 x 2^52 (FP32: 2^23).
+// ---------------------------------------------------------------------------
+template <typename T> struct Trig;
+
+template <> struct Trig<double>
+{
+    typedef double2 Entry;
+    static constexpr int kEntries = 512, kCopies = 8;
+    static constexpr int kSize = kEntries * kCopies;
+    static constexpr double kStepsPerRadian = 81.48733086305042;  // 256 / pi
+    static constexpr double kLimit = 4294967296.0;
+
+    static __device__ __forceinline__ void fill(Entry* table)
+    {
+        for (int j = threadIdx.x; j < kEntries; j += blockDim.x)
+        {
+            double s, c;
+            sincospi((double) j / (kEntries / 2), &s, &c);
+#pragma unroll
+            for (int k = 0; k < kCopies; ++k)
+                table[j * kCopies + k] = make_double2(c, s);
+        }
+    }
+    static __device__ __forceinline__ void sincos(const Entry* table,
+            double u, double* s, double* c)
+    {
+        constexpr double kShift = 6755399441055744.0;  // 1.5 x 2^52
+        constexpr double h = 3.141592653589793 / (kEntries / 2);
+        constexpr double h2 = h * h, h4 = h2 * h2, h6 = h4 * h2;
+        constexpr double s1 = h, s3 = -h * h2 / 6.0, s5 = h * h4 / 120.0;
+        // f2^3 on [0, 1/4] as 3/8 f2^2 - 9/256 f2 (+ 1/2048)
+        constexpr double c4 = h4 / 24.0 - h6 / 720.0 * (3.0 / 8.0);
+        constexpr double c2 = -h2 / 2.0 + h6 / 720.0 * (9.0 / 256.0);
+        const double t = u + kShift;
+        const int n = __double2loint(t);
+        const double f = u - (t - kShift);
+        const double f2 = f * f;
+        const double sr = f * fma(f2, fma(f2, s5, s3), s1);
+        const double cm = f2 * fma(f2, c4, c2);
+        const Entry e = table[((n & (kEntries - 1)) * kCopies) |
+                (threadIdx.x & (kCopies - 1))];
+        *c = fma(e.x, cm, fma(-e.y, sr, e.x));
+        *s = fma(e.y, cm, fma(e.x, sr, e.y));
+    }
+    static __device__ __forceinline__ void exact(double u, double* s,
+            double* c)
+    {
+        sincospi(u * (1.0 / (kEntries / 2)), s, c);
+    }
+    static __device__ __forceinline__ void checked(const Entry* table,
+            double u, double* s, double* c)
+    {
+        if (fabs(u) < kLimit) sincos(table, u, s, c);
+        else exact(u, s, c);
+    }
+};
+
+template <> struct Trig<float>
+{
+    typedef float2 Entry;
+    static constexpr int kEntries = 256, kCopies = 16;
+    static constexpr int kSize = kEntries * kCopies;
+    static constexpr double kStepsPerRadian = 40.74366543152521;  // 128 / pi
+    static constexpr float kLimit = 2097152.0f;
+
+    static __device__ __forceinline__ void fill(Entry* table)
+    {
+        for (int j = threadIdx.x; j < kEntries; j += blockDim.x)
+        {
+            float s, c;
+            sincospif((float) j / (kEntries / 2), &s, &c);
+#pragma unroll
+            for (int k = 0; k < kCopies; ++k)
+                table[j * kCopies + k] = make_float2(c, s);
+        }
+    }
+    // Two phases as a packed pair.
+    static __device__ __forceinline__ void sincos2(const Entry* table,
+            f32x2 u, float* s, float* c)
+    {
+        constexpr float kShift = 12582912.0f;  // 1.5 x 2^23
+        constexpr double h = 3.141592653589793 / (kEntries / 2);
+        constexpr float s1 = (float) h, s3 = (float) (-h * h * h / 6.0);
+        // f2^2 on [0, 1/4] as f2 / 4 (- 1/128)
+        constexpr float c2 = (float) (-h * h / 2.0 + h * h * h * h / 24.0 /
+                4.0);
+        const f32x2 t = add2(u, pack2(kShift, kShift));
+        const f32x2 f = fma2(add2(t, pack2(-kShift, -kShift)),
+                pack2(-1.0f, -1.0f), u);
+        const f32x2 f2 = mul2(f, f);
+        const f32x2 sr2 = mul2(f, fma2(f2, pack2(s3, s3), pack2(s1, s1)));
+        const f32x2 cm2 = mul2(f2, pack2(c2, c2));
+        float tt[2], sr[2], cm[2];
+        unpack2(t, tt[0], tt[1]);
+        unpack2(sr2, sr[0], sr[1]);
+        unpack2(cm2, cm[0], cm[1]);
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+        {
+            const int n = __float_as_int(tt[j]);
+            const Entry e = table[((n & (kEntries - 1)) * kCopies) |
+                    (threadIdx.x & (kCopies - 1))];
+            c[j] = fmaf(e.x, cm[j], fmaf(-e.y, sr[j], e.x));
+            s[j] = fmaf(e.y, cm[j], fmaf(e.x, sr[j], e.y));
+        }
+    }
+    static __device__ __forceinline__ void exact(float u, float* s, float* c)
+    {
+        sincospif(u * (1.0f / (kEntries / 2)), s, c);
+    }
+    static __device__ __forceinline__ void checked(const Entry* table,
+            float u, float* s, float* c)
+    {
+        if (!(fabsf(u) < kLimit))
+        {
+            exact(u, s, c);
+            return;
+        }
+        float s2[2], c2[2];
+        sincos2(table, pack2(u, u), s2, c2);
+        *s = s2[0];
+        *c = c2[0];
+    }
+};
 
 }  // namespace oskb
