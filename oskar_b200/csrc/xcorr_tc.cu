@@ -838,6 +838,10 @@ struct GemmParams
     // adds nothing
     const int* skip_flags = nullptr;
     int* err;
+    // Integer forms: the last wave's tasks split into this many runs each,
+    // whose partial sums go to partial (1: every task whole).
+    int pieces = 1;
+    uint32_t* partial = nullptr;
     // Auto-correlations (optional): the diagonal station pairs of the
     // diagonal tiles, V_pp = J_p B J_p^H, added into
     // autos[(g * num_st + p) * 8 + 2 x 2] for global problem g; NULL: none.
@@ -1925,12 +1929,124 @@ constexpr size_t gemm_i8_smem_bytes()
     return 1024 + (size_t) kI8Stages * kI8StageBytes + sizeof(I8Ctl);
 }
 
+// ---------------------------------------------------------------------------
+// Work split of the integer contractions. A task (problem, tile) is a run of
+// k blocks; tasks go to the CTAs in turn. When the last, incomplete wave (all
+// tasks when a call has fewer than CTAs) leaves at least half of the CTAs
+// idle, each of its R tasks is split into S = CTAs / R runs of k blocks, run
+// i of every task at a time side by side (so that the tasks still share their
+// operand blocks in L2: equal shares that start anywhere in a task measured 4
+// % slower than no split on a block of 300 stations, with HBM as the bound).
+// The runs' sums go to partial slots and a second kernel adds the slots of
+// each task and stores the visibilities. The sums are exact integers over all
+// k blocks (Sum96, and 128 bits in the six-limb form), so the result does not
+// depend, to the last bit, on how the tasks were split. 256 stations x 20,000
+// sources, six limbs (72 tasks on 148 SMs, S = 2): 1,136 -> 693 us a call; 64
+// stations x 3,000 sources x 8 problems, three limbs (24 tasks, S = 6): 126 ->
+// 112 us.
+// ---------------------------------------------------------------------------
+struct TaskRun
+{
+    int task, kb0, kb1;
+    int slot;   // -1: a whole task; else the partial slot
+};
+
+struct TaskWalk
+{
+    int next, full, rest, pieces, nkb, ctas;
+    __device__ __forceinline__ TaskWalk(const GemmParams& prm, int ntasks,
+            int nkb_)
+            : next(blockIdx.x), pieces(prm.pieces), nkb(nkb_),
+              ctas(gridDim.x)
+    {
+        rest = pieces > 1 ? ntasks % ctas : 0;
+        full = ntasks - rest;
+    }
+    __device__ __forceinline__ bool operator()(TaskRun& r)
+    {
+        if (next < full)
+        {
+            r.task = next;
+            r.kb0 = 0;
+            r.kb1 = nkb;
+            r.slot = -1;
+            next += ctas;
+            return true;
+        }
+        // next - full runs over the CTAs once
+        const int c = next - full;
+        if (c >= rest * pieces) return false;
+        const int k = c % rest, i = c / rest;
+        r.task = full + k;
+        r.kb0 = (int) ((long long) nkb * i / pieces);
+        r.kb1 = (int) ((long long) nkb * (i + 1) / pieces);
+        r.slot = c;
+        next = full + rest * pieces;
+        return true;
+    }
+};
+
+// Partial slots: WORDS words x 256 epilogue threads each; slot i R + k holds
+// run i of last-wave task k.
+template <int WORDS>
+__device__ __forceinline__ uint32_t* partial_slot(uint32_t* partial, int slot)
+{
+    return partial + (size_t) slot * WORDS * 256;
+}
+
+// Exact sums of one chunk's 64-bit integers at the chunk's scale 2^-2b, in
+// units of 2^-2 (kI8Buckets - 1): 96 bits (a chunk's integer is below 2^49,
+// the shift at most 30, so 2^16 chunks fit).
+struct Sum96
+{
+    uint32_t w[3];
+    __device__ __forceinline__ void clear() { w[0] = w[1] = w[2] = 0; }
+    __device__ __forceinline__ void add(uint32_t a0, uint32_t a1,
+            uint32_t a2)
+    {
+        asm("add.cc.u32 %0, %0, %3;\n\t"
+            "addc.cc.u32 %1, %1, %4;\n\t"
+            "addc.u32 %2, %2, %5;"
+            : "+r"(w[0]), "+r"(w[1]), "+r"(w[2])
+            : "r"(a0), "r"(a1), "r"(a2));
+    }
+    __device__ __forceinline__ void add_shifted(long long v, int shift)
+    {
+        const uint32_t lo = (uint32_t) v, hi = (uint32_t) (v >> 32);
+        const uint32_t sign = (uint32_t) ((int) hi >> 31);
+        add(lo << shift, __funnelshift_l(lo, hi, shift),
+                __funnelshift_l(hi, sign, shift));
+    }
+    // rounded to FP64 from the magnitude (relative error 2^-52)
+    __device__ __forceinline__ double value() const
+    {
+        const bool neg = (int) w[2] < 0;
+        uint32_t a0 = w[0], a1 = w[1], a2 = w[2];
+        if (neg)
+        {
+            a0 = ~a0;
+            a1 = ~a1;
+            a2 = ~a2;
+            asm("add.cc.u32 %0, %0, 1;\n\t"
+                "addc.cc.u32 %1, %1, 0;\n\t"
+                "addc.u32 %2, %2, 0;" : "+r"(a0), "+r"(a1), "+r"(a2));
+        }
+        const double v = (double) a2 * 18446744073709551616.0 +
+                (double) (((unsigned long long) a1 << 32) | a0);
+        return neg ? -v : v;
+    }
+};
+
+constexpr int kI8ShiftMax = 2 * (kI8Buckets - 1);
+// units of the exact sums against those of the limb products
+constexpr double kI8SumUnit = 1.0 / (1 << kI8ShiftMax);
+
 // One drain of the three integer accumulators over this thread's 64
-// columns (taddr): (D0 2^16 + D1 2^8 + D2) scale per column (exact before
-// the scale, |.| < 2^48), folded into the Re V and Im V sums of its 16
-// column stations.
-__device__ __forceinline__ void i8_drain64(uint32_t taddr, int c,
-        double scale, double (&accR)[16], double (&accI)[16])
+// columns (taddr): D0 2^16 + D1 2^8 + D2 per column (|.| < 2^48), folded
+// into the Re V and Im V sums of its 16 column stations at the chunk's
+// scale.
+__device__ __forceinline__ void i8_drain64(uint32_t taddr, int c, int shift,
+        Sum96 (&accR)[16], Sum96 (&accI)[16])
 {
 #pragma unroll
     for (int j0 = 0; j0 < 64; j0 += 16)
@@ -1940,31 +2056,32 @@ __device__ __forceinline__ void i8_drain64(uint32_t taddr, int c,
         ptx::tmem_ld16(taddr + 128 + j0, v1);
         ptx::tmem_ld16(taddr + 256 + j0, v2);
         ptx::tmem_ld_wait();
-        double v[16];
-#pragma unroll
-        for (int j = 0; j < 16; ++j)
-            v[j] = ((double) (int) v0[j] * 65536.0 +
-                    (double) (int) v1[j] * 256.0 +
-                    (double) (int) v2[j]) * scale;
         // Re V = G00 + G11, Im V = G10 - G01 across the row pair
         // (lanes l, l ^ 1), as the FP16 kernels fold
 #pragma unroll
         for (int qq = 0; qq < 4; ++qq)
         {
-            const int jb = 4 * qq;
-            const double s0 = c ? v[jb + 0] : v[jb + 2];
-            const double s1 = c ? v[jb + 1] : v[jb + 3];
-            const double r0 = __shfl_xor_sync(0xffffffffu, s0, 1);
-            const double r1 = __shfl_xor_sync(0xffffffffu, s1, 1);
-            const double g00 = c ? r0 : v[jb + 0];
-            const double g01 = c ? r1 : v[jb + 1];
-            const double g10 = c ? v[jb + 2] : r0;
-            const double g11 = c ? v[jb + 3] : r1;
-            accR[j0 / 4 + qq] += g00 + g11;
-            accI[j0 / 4 + qq] += g10 - g01;
+            long long v[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                v[j] = (long long) (int) v0[4 * qq + j] * 65536 +
+                        (long long) (int) v1[4 * qq + j] * 256 +
+                        (int) v2[4 * qq + j];
+            const long long s0 = c ? v[0] : v[2];
+            const long long s1 = c ? v[1] : v[3];
+            const long long r0 = __shfl_xor_sync(0xffffffffu, s0, 1);
+            const long long r1 = __shfl_xor_sync(0xffffffffu, s1, 1);
+            const long long g00 = c ? r0 : v[0];
+            const long long g01 = c ? r1 : v[1];
+            const long long g10 = c ? v[2] : r0;
+            const long long g11 = c ? v[3] : r1;
+            accR[j0 / 4 + qq].add_shifted(g00 + g11, shift);
+            accI[j0 / 4 + qq].add_shifted(g10 - g01, shift);
         }
     }
 }
+
+constexpr int kI8PartialWords = 96;   // 32 sums of three words
 
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_i8_kernel(const GemmParams prm)
@@ -2002,6 +2119,8 @@ gemm_i8_kernel(const GemmParams prm)
     const int ntasks = ntile * prm.num_problems;
     const int nkb_used = prm.i8_counts[0];
     const int nchunk = prm.i8_counts[1];
+    TaskWalk walk(prm, ntasks, nkb_used);
+    TaskRun run;
 
     if (warp == 0)
     {
@@ -2013,15 +2132,14 @@ gemm_i8_kernel(const GemmParams prm)
             int stage = 0;
             uint32_t phase = 0;
             uint32_t issued = 0, issued_par = 0;  // bit s: stage s
-            for (int task = blockIdx.x; task < ntasks && !*abort;
-                    task += gridDim.x)
+            while (!*abort && walk(run))
             {
-                const int prob = task / ntile;
+                const int prob = run.task / ntile;
                 int rb, cb;
-                tile_of(task - prob * ntile, rb, cb);
+                tile_of(run.task - prob * ntile, rb, cb);
                 const bool diag = rb == cb;
                 const uint8_t* img = prm.W + (size_t) prob * prm.image_stride;
-                for (int kb = 0; kb < nkb_used; ++kb)
+                for (int kb = run.kb0; kb < run.kb1; ++kb)
                 {
                     if (!ptx::mbar_wait(&ctl->empty[stage], phase ^ 1,
                             prm.err, 31, abort))
@@ -2058,15 +2176,17 @@ gemm_i8_kernel(const GemmParams prm)
             int stage = 0;
             uint32_t phase = 0, dpar = 0;
             bool ok = true;
-            for (int task = blockIdx.x; task < ntasks && ok;
-                    task += gridDim.x)
+            while (ok && walk(run))
             {
-                const int prob = task / ntile;
+                const int prob = run.task / ntile;
                 int rb, cb;
-                tile_of(task - prob * ntile, rb, cb);
+                tile_of(run.task - prob * ntile, rb, cb);
                 const bool diag = rb == cb;
                 for (int ch = 0; ch < nchunk && ok; ++ch)
                 {
+                    const int kb0 = max(prm.i8_chunk_kb[ch], run.kb0);
+                    const int kb1 = min(prm.i8_chunk_kb[ch + 1], run.kb1);
+                    if (kb0 >= kb1) continue;
                     // the epilogue has read the accumulators' last sums
                     if (!ptx::mbar_wait(&ctl->dempty, dpar ^ 1, prm.err, 33,
                             abort))
@@ -2075,8 +2195,6 @@ gemm_i8_kernel(const GemmParams prm)
                         break;
                     }
                     ptx::tc_fence_after();
-                    const int kb0 = prm.i8_chunk_kb[ch];
-                    const int kb1 = prm.i8_chunk_kb[ch + 1];
                     for (int kb = kb0; kb < kb1; ++kb)
                     {
                         if (!ptx::mbar_wait(&ctl->full[stage], phase, prm.err,
@@ -2139,18 +2257,21 @@ gemm_i8_kernel(const GemmParams prm)
                 (uint32_t) (64 * h);
         uint32_t dpar = 0;
         bool ok = true;
-        for (int task = blockIdx.x; task < ntasks && ok; task += gridDim.x)
+        while (ok && walk(run))
         {
-            const int prob = task / ntile;
-            int rb, cb;
-            tile_of(task - prob * ntile, rb, cb);
-            // sums of Re V and Im V, in units of 2^16 / q^2, of the
-            // thread's 16 column stations
-            double accR[16], accI[16];
+            // sums of Re V and Im V of the thread's 16 column stations
+            Sum96 accR[16], accI[16];
 #pragma unroll
-            for (int j = 0; j < 16; ++j) accR[j] = accI[j] = 0.0;
+            for (int j = 0; j < 16; ++j)
+            {
+                accR[j].clear();
+                accI[j].clear();
+            }
             for (int ch = 0; ch < nchunk; ++ch)
             {
+                if (max(prm.i8_chunk_kb[ch], run.kb0) >=
+                        min(prm.i8_chunk_kb[ch + 1], run.kb1))
+                    continue;
                 if (!ptx::mbar_wait(&ctl->dfull, dpar, prm.err, 36, abort))
                 {
                     ok = false;
@@ -2158,19 +2279,42 @@ gemm_i8_kernel(const GemmParams prm)
                 }
                 ptx::tc_fence_after();
                 // the chunk's bucket b: its entries carry q 2^b each
-                i8_drain64(taddr, c, ldexp(1.0, -2 * prm.i8_chunk_bucket[ch]),
-                        accR, accI);
+                i8_drain64(taddr, c, kI8ShiftMax - 2 *
+                        prm.i8_chunk_bucket[ch], accR, accI);
                 ptx::tc_fence_before();
                 __syncwarp();
                 if (lane == 0) ptx::mbar_arrive(&ctl->dempty);
                 dpar ^= 1;
             }
             if (!ok) break;
-            const int g = prm.prob0 + prob;
+            if (run.slot >= 0)
+            {
+                uint32_t* o = partial_slot<kI8PartialWords>(prm.partial,
+                        run.slot) + (threadIdx.x - 64);
+#pragma unroll
+                for (int j = 0; j < 16; ++j)
+#pragma unroll
+                    for (int k = 0; k < 3; ++k)
+                    {
+                        o[(6 * j + k) * 256] = accR[j].w[k];
+                        o[(6 * j + 3 + k) * 256] = accI[j].w[k];
+                    }
+                continue;
+            }
+            const int prob = run.task / ntile;
+            int rb, cb;
+            tile_of(run.task - prob * ntile, rb, cb);
             const double q = (double) i8_scale_from_bits(
-                    prm.maxabs_bits[prm.maxabs_stride * g]);
-            square_task_store(prm, accR, accI, 65536.0 / (q * q), row, h,
-                    prob, rb, cb);
+                    prm.maxabs_bits[prm.maxabs_stride * (prm.prob0 + prob)]);
+            const double unit = 65536.0 * kI8SumUnit / (q * q);
+#pragma unroll
+            for (int j = 0; j < 16; ++j)
+            {
+                const double re[1] = {accR[j].value()};
+                const double im[1] = {accI[j].value()};
+                task_store<1>(prm, re, im, unit, row, 16 * h + j, prob, rb,
+                        cb);
+            }
         }
     }
 
@@ -2178,6 +2322,38 @@ gemm_i8_kernel(const GemmParams prm)
     __syncthreads();
     ptx::tc_fence_after();
     if (warp == 1) ptx::tmem_dealloc(tmem, kI8TmemCols);
+}
+
+// Last-wave tasks of gemm_i8_kernel: block (k, j) adds the partial sums of
+// last-wave task k's column station j of each epilogue thread and stores
+// them.
+__global__ void __launch_bounds__(256)
+fixup_i8_kernel(const GemmParams prm)
+{
+    if (*prm.err != 0) return;   // a wait expired: sums incomplete
+    if (prm.skip_flags && (*prm.skip_flags & 1)) return;
+    const int ntile = prm.nrb * (prm.nrb + 1) / 2;
+    const int k = blockIdx.x, j = blockIdx.y, rest = gridDim.x;
+    Sum96 r, i;
+    r.clear();
+    i.clear();
+    for (int n = 0; n < prm.pieces; ++n)
+    {
+        const uint32_t* v = partial_slot<kI8PartialWords>(prm.partial,
+                n * rest + k) + (size_t) 6 * j * 256 + threadIdx.x;
+        r.add(v[0], v[256], v[512]);
+        i.add(v[768], v[1024], v[1280]);
+    }
+    const int warp = (threadIdx.x >> 5) + 2, lane = threadIdx.x & 31;
+    const int row = 32 * (warp & 3) + lane, h = (warp - 2) >> 2;
+    const int task = ntile * prm.num_problems - rest + k, prob = task / ntile;
+    int rb, cb;
+    tile_of(task - prob * ntile, rb, cb);
+    const double q = (double) i8_scale_from_bits(
+            prm.maxabs_bits[prm.maxabs_stride * (prm.prob0 + prob)]);
+    const double re[1] = {r.value()}, im[1] = {i.value()};
+    task_store<1>(prm, re, im, 65536.0 * kI8SumUnit / (q * q), row,
+            16 * h + j, prob, rb, cb);
 }
 
 // ===========================================================================
@@ -2403,58 +2579,65 @@ constexpr size_t gemm_l6_smem_bytes()
     return 1024 + (size_t) kL6Stages * kL6StageBytes + sizeof(L6Ctl);
 }
 
-// One drain of the six accumulators over this thread's 32 columns (taddr,
-// 64 columns per accumulator): sum_c D_c 2^(8 (5 - c)) scale per column,
-// folded into the Re V and Im V sums of its 8 column stations.
-__device__ __forceinline__ void l6_drain32(uint32_t taddr, int c,
-        double scale, double (&accR)[8], double (&accI)[8])
+// Exact 128-bit sums of the six-limb form: a chunk's integer is below 2^73,
+// the bucket shift at most 30, so 2^24 chunks fit.
+typedef __int128 Sum128;
+
+__device__ __forceinline__ double sum_value(Sum128 v)
 {
+    // rounded to FP64 from the magnitude (relative error 2^-52)
+    const bool neg = v < 0;
+    const unsigned __int128 a = neg ? -(unsigned __int128) v :
+            (unsigned __int128) v;
+    const double d = (double) (unsigned long long) (a >> 64) *
+            18446744073709551616.0 + (double) (unsigned long long) a;
+    return neg ? -d : d;
+}
+
+// One drain of the six accumulators over this thread's 32 columns (taddr,
+// 64 columns per accumulator): sum_c D_c 2^(8 (5 - c)) per column, as a
+// high part in units of 2^24 (D0 .. D2) and a low part (D3 .. D5), folded
+// into the Re V and Im V sums of its 8 column stations at the chunk's scale.
+__device__ __forceinline__ void l6_drain32(uint32_t taddr, int c, int shift,
+        Sum128 (&accR)[8], Sum128 (&accI)[8])
+{
+#pragma unroll 1
+    for (int part = 0; part < 2; ++part)
 #pragma unroll
-    for (int j0 = 0; j0 < 32; j0 += 16)
-    {
-        double v[16];
+        for (int j0 = 0; j0 < 32; j0 += 16)
         {
             uint32_t u0[16], u1[16], u2[16];
-            ptx::tmem_ld16(taddr + j0, u0);
-            ptx::tmem_ld16(taddr + 64 + j0, u1);
-            ptx::tmem_ld16(taddr + 128 + j0, u2);
+            ptx::tmem_ld16(taddr + 192 * part + j0, u0);
+            ptx::tmem_ld16(taddr + 192 * part + 64 + j0, u1);
+            ptx::tmem_ld16(taddr + 192 * part + 128 + j0, u2);
             ptx::tmem_ld_wait();
+            const int sh = shift + (part ? 0 : 24);
+            // Re V = G00 + G11, Im V = G10 - G01 across the row pair
+            // (lanes l, l ^ 1), as i8_drain64
 #pragma unroll
-            for (int j = 0; j < 16; ++j)
-                v[j] = ((double) (int) u0[j] * 256.0 + (double) (int) u1[j])
-                        * 256.0 + (double) (int) u2[j];
-        }
-        {
-            uint32_t u3[16], u4[16], u5[16];
-            ptx::tmem_ld16(taddr + 192 + j0, u3);
-            ptx::tmem_ld16(taddr + 256 + j0, u4);
-            ptx::tmem_ld16(taddr + 320 + j0, u5);
-            ptx::tmem_ld_wait();
+            for (int qq = 0; qq < 4; ++qq)
+            {
+                long long v[4];
 #pragma unroll
-            for (int j = 0; j < 16; ++j)
-                v[j] = (((v[j] * 256.0 + (double) (int) u3[j]) * 256.0 +
-                        (double) (int) u4[j]) * 256.0 +
-                        (double) (int) u5[j]) * scale;
+                for (int j = 0; j < 4; ++j)
+                    v[j] = (long long) (int) u0[4 * qq + j] * 65536 +
+                            (long long) (int) u1[4 * qq + j] * 256 +
+                            (int) u2[4 * qq + j];
+                const long long s0 = c ? v[0] : v[2];
+                const long long s1 = c ? v[1] : v[3];
+                const long long r0 = __shfl_xor_sync(0xffffffffu, s0, 1);
+                const long long r1 = __shfl_xor_sync(0xffffffffu, s1, 1);
+                const long long g00 = c ? r0 : v[0];
+                const long long g01 = c ? r1 : v[1];
+                const long long g10 = c ? v[2] : r0;
+                const long long g11 = c ? v[3] : r1;
+                accR[j0 / 4 + qq] += (Sum128) (g00 + g11) << sh;
+                accI[j0 / 4 + qq] += (Sum128) (g10 - g01) << sh;
+            }
         }
-        // Re V = G00 + G11, Im V = G10 - G01 across the row pair
-        // (lanes l, l ^ 1), as i8_drain64
-#pragma unroll
-        for (int qq = 0; qq < 4; ++qq)
-        {
-            const int jb = 4 * qq;
-            const double s0 = c ? v[jb + 0] : v[jb + 2];
-            const double s1 = c ? v[jb + 1] : v[jb + 3];
-            const double r0 = __shfl_xor_sync(0xffffffffu, s0, 1);
-            const double r1 = __shfl_xor_sync(0xffffffffu, s1, 1);
-            const double g00 = c ? r0 : v[jb + 0];
-            const double g01 = c ? r1 : v[jb + 1];
-            const double g10 = c ? v[jb + 2] : r0;
-            const double g11 = c ? v[jb + 3] : r1;
-            accR[j0 / 4 + qq] += g00 + g11;
-            accI[j0 / 4 + qq] += g10 - g01;
-        }
-    }
 }
+
+constexpr int kL6PartialWords = 64;   // 16 sums of four words
 
 // Tasks: (problem, square tile (rb <= cb), column half); 2 per tile.
 __global__ void __launch_bounds__(kGemmThreads, 1)
@@ -2493,6 +2676,8 @@ gemm_l6_kernel(const GemmParams prm)
     const int ntasks = ntile * prm.num_problems;
     const int nkb_used = prm.i8_counts[0];
     const int nchunk = prm.i8_counts[1];
+    TaskWalk walk(prm, ntasks, nkb_used);
+    TaskRun run;
 
     if (warp == 0)
     {
@@ -2505,17 +2690,16 @@ gemm_l6_kernel(const GemmParams prm)
             int stage = 0;
             uint32_t phase = 0;
             uint32_t issued = 0, issued_par = 0;  // bit s: stage s
-            for (int task = blockIdx.x; task < ntasks && !*abort;
-                    task += gridDim.x)
+            while (!*abort && walk(run))
             {
-                const int prob = task / ntile;
-                const int tt = task - prob * ntile;
+                const int prob = run.task / ntile;
+                const int tt = run.task - prob * ntile;
                 const int half = tt & 1;
                 int rb, cb;
                 tile_of(tt >> 1, rb, cb);
                 const bool diag = rb == cb;
                 const uint8_t* img = prm.W + (size_t) prob * prm.image_stride;
-                for (int kb = 0; kb < nkb_used; ++kb)
+                for (int kb = run.kb0; kb < run.kb1; ++kb)
                 {
                     if (!ptx::mbar_wait(&ctl->empty[stage], phase ^ 1,
                             prm.err, 51, abort))
@@ -2560,17 +2744,19 @@ gemm_l6_kernel(const GemmParams prm)
             int stage = 0;
             uint32_t phase = 0, dpar = 0;
             bool ok = true;
-            for (int task = blockIdx.x; task < ntasks && ok;
-                    task += gridDim.x)
+            while (ok && walk(run))
             {
-                const int prob = task / ntile;
-                const int tt = task - prob * ntile;
+                const int prob = run.task / ntile;
+                const int tt = run.task - prob * ntile;
                 const int half = tt & 1;
                 int rb, cb;
                 tile_of(tt >> 1, rb, cb);
                 const bool diag = rb == cb;
                 for (int ch = 0; ch < nchunk && ok; ++ch)
                 {
+                    const int kb0 = max(prm.i8_chunk_kb[ch], run.kb0);
+                    const int kb1 = min(prm.i8_chunk_kb[ch + 1], run.kb1);
+                    if (kb0 >= kb1) continue;
                     // the epilogue has read the accumulators' last sums
                     if (!ptx::mbar_wait(&ctl->dempty, dpar ^ 1, prm.err, 53,
                             abort))
@@ -2579,8 +2765,6 @@ gemm_l6_kernel(const GemmParams prm)
                         break;
                     }
                     ptx::tc_fence_after();
-                    const int kb0 = prm.i8_chunk_kb[ch];
-                    const int kb1 = prm.i8_chunk_kb[ch + 1];
                     for (int kb = kb0; kb < kb1; ++kb)
                     {
                         if (!ptx::mbar_wait(&ctl->full[stage], phase, prm.err,
@@ -2662,18 +2846,16 @@ gemm_l6_kernel(const GemmParams prm)
                 (uint32_t) (32 * h);
         uint32_t dpar = 0;
         bool ok = true;
-        for (int task = blockIdx.x; task < ntasks && ok; task += gridDim.x)
+        while (ok && walk(run))
         {
-            const int prob = task / ntile;
-            const int tt = task - prob * ntile;
-            const int half = tt & 1;
-            int rb, cb;
-            tile_of(tt >> 1, rb, cb);
-            double accR[8], accI[8];
+            Sum128 accR[8], accI[8];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) accR[j] = accI[j] = 0.0;
+            for (int j = 0; j < 8; ++j) accR[j] = accI[j] = 0;
             for (int ch = 0; ch < nchunk; ++ch)
             {
+                if (max(prm.i8_chunk_kb[ch], run.kb0) >=
+                        min(prm.i8_chunk_kb[ch + 1], run.kb1))
+                    continue;
                 if (!ptx::mbar_wait(&ctl->dfull, dpar, prm.err, 56, abort))
                 {
                     ok = false;
@@ -2681,19 +2863,45 @@ gemm_l6_kernel(const GemmParams prm)
                 }
                 ptx::tc_fence_after();
                 // the chunk's bucket b: its entries carry q 2^b each
-                l6_drain32(taddr, c, ldexp(1.0, -2 * prm.i8_chunk_bucket[ch]),
-                        accR, accI);
+                l6_drain32(taddr, c, kI8ShiftMax - 2 *
+                        prm.i8_chunk_bucket[ch], accR, accI);
                 ptx::tc_fence_before();
                 __syncwarp();
                 if (lane == 0) ptx::mbar_arrive(&ctl->dempty);
                 dpar ^= 1;
             }
             if (!ok) break;
-            const int g = prm.prob0 + prob;
+            if (run.slot >= 0)
+            {
+                uint32_t* o = partial_slot<kL6PartialWords>(prm.partial,
+                        run.slot) + (threadIdx.x - 64);
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+                    {
+                        o[(8 * j + k) * 256] = (uint32_t) ((unsigned __int128)
+                                accR[j] >> (32 * k));
+                        o[(8 * j + 4 + k) * 256] = (uint32_t) (
+                                (unsigned __int128) accI[j] >> (32 * k));
+                    }
+                continue;
+            }
+            const int prob = run.task / ntile;
+            const int tt = run.task - prob * ntile;
+            int rb, cb;
+            tile_of(tt >> 1, rb, cb);
             const double q = l6_scale_from_bits(
-                    prm.maxabs_bits[prm.maxabs_stride * g]);
-            task_store<8>(prm, accR, accI, 1099511627776.0 / (q * q), row,
-                    16 * half + 8 * h, prob, rb, cb);
+                    prm.maxabs_bits[prm.maxabs_stride * (prm.prob0 + prob)]);
+            const double unit = 1099511627776.0 * kI8SumUnit / (q * q);
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+            {
+                const double re[1] = {sum_value(accR[j])};
+                const double im[1] = {sum_value(accI[j])};
+                task_store<1>(prm, re, im, unit, row, 16 * (tt & 1) + 8 * h +
+                        j, prob, rb, cb);
+            }
         }
     }
 
@@ -2701,6 +2909,43 @@ gemm_l6_kernel(const GemmParams prm)
     __syncthreads();
     ptx::tc_fence_after();
     if (warp == 1) ptx::tmem_dealloc(tmem, kL6TmemCols);
+}
+
+// Last-wave tasks of gemm_l6_kernel, as fixup_i8_kernel.
+__global__ void __launch_bounds__(256)
+fixup_l6_kernel(const GemmParams prm)
+{
+    if (*prm.err != 0) return;   // a wait expired: sums incomplete
+    if (prm.skip_flags && (*prm.skip_flags & 1)) return;
+    const int ntile = prm.nrb * (prm.nrb + 1);
+    const int k = blockIdx.x, j = blockIdx.y, rest = gridDim.x;
+    unsigned __int128 r = 0, i = 0;
+    for (int n = 0; n < prm.pieces; ++n)
+    {
+        const uint32_t* v = partial_slot<kL6PartialWords>(prm.partial,
+                n * rest + k) + (size_t) 8 * j * 256 + threadIdx.x;
+        unsigned __int128 a = 0, b = 0;
+#pragma unroll
+        for (int w = 0; w < 4; ++w)
+        {
+            a |= (unsigned __int128) v[256 * w] << (32 * w);
+            b |= (unsigned __int128) v[1024 + 256 * w] << (32 * w);
+        }
+        r += a;
+        i += b;
+    }
+    const int warp = (threadIdx.x >> 5) + 2, lane = threadIdx.x & 31;
+    const int row = 32 * (warp & 3) + lane, h = (warp - 2) >> 2;
+    const int task = ntile * prm.num_problems - rest + k, prob = task / ntile;
+    const int tt = task - prob * ntile;
+    int rb, cb;
+    tile_of(tt >> 1, rb, cb);
+    const double q = l6_scale_from_bits(
+            prm.maxabs_bits[prm.maxabs_stride * (prm.prob0 + prob)]);
+    const double re[1] = {sum_value((Sum128) r)};
+    const double im[1] = {sum_value((Sum128) i)};
+    task_store<1>(prm, re, im, 1099511627776.0 * kI8SumUnit / (q * q), row,
+            16 * (tt & 1) + 8 * h + j, prob, rb, cb);
 }
 
 // FP32 entry point helpers: station u, v widened to FP64; the FP64 sums
@@ -2979,7 +3224,77 @@ cudaEvent_t timing_start(cudaStream_t stream)
     return g_ev[g_ev_used++].second;
 }
 
-int launch_gemm(GemmParams& gp, cudaStream_t stream)
+// Room for the partial sums of a split last wave: the tail of the caller's
+// workspace where it is large enough, else the library's scratch pool (not
+// while the stream is captured, and not for the allocation-free entry
+// point), else none: the last wave's tasks then run whole, with the same
+// results to the last bit.
+struct PartialRoom
+{
+    uint8_t* tail = nullptr;
+    size_t tail_bytes = 0;
+    bool pool = true;
+};
+
+// Launches an integer contraction (gemm, and fixup for a split last wave;
+// sums_per_thread: the fixup's grid height, words: of a partial slot per
+// thread) of ntasks tasks of at most nkb k blocks, kb_us microseconds each.
+// The last wave is split when that saves more than the ~15 us of the partial
+// sums and the second launch, into runs of at least four k blocks.
+int launch_integer(void (*gemm)(GemmParams), size_t smem,
+        void (*fixup)(GemmParams), int sums_per_thread, int words,
+        double kb_us, GemmParams& gp, long long ntasks,
+        const PartialRoom& room, cudaStream_t stream)
+{
+    const int sms = num_sms();
+    const int rest = (int) (ntasks % sms);
+    void* to_free = nullptr;
+    gp.pieces = rest > 0 ? std::max(1, std::min(sms / rest, gp.nkb / 4)) : 1;
+    gp.partial = nullptr;
+    if ((1.0 - 1.0 / gp.pieces) * gp.nkb * kb_us > 15.0)
+    {
+        const size_t need = (size_t) rest * gp.pieces * words * 256 *
+                sizeof(uint32_t);
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        if (room.tail_bytes >= need)
+            gp.partial = reinterpret_cast<uint32_t*>(room.tail);
+        else if (room.pool && cudaStreamIsCapturing(stream, &cs) ==
+                cudaSuccess && cs == cudaStreamCaptureStatusNone)
+        {
+            if (scratch_alloc(&to_free, need, stream) == cudaSuccess)
+                gp.partial = reinterpret_cast<uint32_t*>(to_free);
+            else
+            {
+                to_free = nullptr;
+                cudaGetLastError();
+            }
+        }
+    }
+    if (!gp.partial) gp.pieces = 1;
+    const int grid = gp.partial || ntasks >= sms ? sms : (int) ntasks;
+    cudaEvent_t ev_stop = timing_start(stream);
+    gemm<<<grid, kGemmThreads, smem, stream>>>(gp);
+    int err = check_launch("tc gemm (integer)");
+    if (!err && gp.partial)
+    {
+        fixup<<<dim3(rest, sums_per_thread), 256, 0, stream>>>(gp);
+        err = check_launch("tc gemm (integer, last wave)");
+    }
+    if (ev_stop) cudaEventRecord(ev_stop, stream);
+    if (to_free) scratch_free(to_free, stream);
+    return err;
+}
+
+int launch_gemm_l6(GemmParams& gp, const PartialRoom& room,
+        cudaStream_t stream)
+{
+    return launch_integer(gemm_l6_kernel, gemm_l6_smem_bytes(),
+            fixup_l6_kernel, 8, kL6PartialWords, 1.8, gp, (long long) gp.nrb * (gp.nrb + 1) *
+            gp.num_problems, room, stream);
+}
+
+int launch_gemm(GemmParams& gp, cudaStream_t stream,
+        const PartialRoom& room = PartialRoom())
 {
     bool wide_fits = false, pair_fits = false;
     const int serr = device_setup(wide_fits, pair_fits);
@@ -2990,13 +3305,10 @@ int launch_gemm(GemmParams& gp, cudaStream_t stream)
     {
         // square tiles (the integer image's only shape)
         g_last_arith.store(8);
-        const int grid = (int) (square < num_sms() ? square : num_sms());
         g_last_tile.store(128);
-        cudaEvent_t ev_stop = timing_start(stream);
-        gemm_i8_kernel<<<grid, kGemmThreads, gemm_i8_smem_bytes(), stream>>>(
-                gp);
-        if (ev_stop) cudaEventRecord(ev_stop, stream);
-        return check_launch("tc gemm (integer)");
+        return launch_integer(gemm_i8_kernel, gemm_i8_smem_bytes(),
+                fixup_i8_kernel, 16, kI8PartialWords, 0.72, gp, square, room,
+                stream);
     }
     const long long wide_n = (long long) wide_tiles(gp.nrb) *
             gp.num_problems;
@@ -3107,7 +3419,8 @@ int jones_block(int casa, int num_sources, int num_stations, int offset_out,
         const double* jones, const double* I, const double* Q,
         const double* U, const double* V, const double* station_u,
         const double* station_v, double uv_min_lambda, double uv_max_lambda,
-        double inv_wavelength, double* vis, uint8_t* ws, cudaStream_t s)
+        double inv_wavelength, double* vis, uint8_t* ws, cudaStream_t s,
+        bool pool = true)
 {
     Header* hdr = reinterpret_cast<Header*>(ws);
     // the status words start at zero; the image is rewritten
@@ -3164,7 +3477,9 @@ int jones_block(int casa, int num_sources, int num_stations, int offset_out,
     gp.inv_wavelength = nullptr; gp.kw_scalar = inv_wavelength;
     gp.uv_min = uv_min_lambda; gp.uv_max = uv_max_lambda;
     gp.casa = casa; gp.err = &hdr->err; gp.autos = nullptr;
-    return launch_gemm(gp, s);
+    PartialRoom room;
+    room.pool = pool;
+    return launch_gemm(gp, s, room);
 }
 
 // Workspace of the FP64-class form: Header, source-order tables (chunks of
@@ -3218,12 +3533,7 @@ int l6_block(int casa, int num_sources, int num_stations, int offset_out,
     gp.inv_wavelength = nullptr; gp.kw_scalar = inv_wavelength;
     gp.uv_min = uv_min_lambda; gp.uv_max = uv_max_lambda;
     gp.casa = casa; gp.err = &hdr->err; gp.autos = nullptr;
-    const long long ntasks = (long long) nrb * (nrb + 1);
-    const int grid = (int) (ntasks < num_sms() ? ntasks : num_sms());
-    cudaEvent_t ev_stop = timing_start(s);
-    gemm_l6_kernel<<<grid, kGemmThreads, gemm_l6_smem_bytes(), s>>>(gp);
-    if (ev_stop) cudaEventRecord(ev_stop, s);
-    return check_launch("tc64 gemm");
+    return launch_gemm_l6(gp, PartialRoom(), s);
 }
 
 // Workspace of the FP32 entry point: Header, order tables, the integer
@@ -3379,12 +3689,7 @@ int correlate_block_l6(int casa, int num_sources, int num_stations,
         gp.inv_wavelength = inv_wavelength; gp.kw_scalar = 0.0;
         gp.uv_min = uv_min_lambda; gp.uv_max = uv_max_lambda;
         gp.casa = casa; gp.err = &hdr->err; gp.autos = autos;
-        const long long ntasks = (long long) nrb * (nrb + 1) * np;
-        const int grid = (int) (ntasks < num_sms() ? ntasks : num_sms());
-        cudaEvent_t ev_stop = timing_start(s);
-        gemm_l6_kernel<<<grid, kGemmThreads, gemm_l6_smem_bytes(), s>>>(gp);
-        if (ev_stop) cudaEventRecord(ev_stop, s);
-        if ((err = check_launch("tc64 gemm"))) return err;
+        if ((err = launch_gemm_l6(gp, PartialRoom(), s))) return err;
     }
     return 0;
 }
@@ -3701,7 +4006,11 @@ int correlate_block(int casa, int num_sources, int num_stations,
         gp.inv_wavelength = inv_wavelength; gp.kw_scalar = 0.0;
         gp.uv_min = uv_min_lambda; gp.uv_max = uv_max_lambda;
         gp.casa = casa; gp.err = &hdr->err; gp.autos = autos;
-        if ((err = launch_gemm(gp, s))) return err;
+        PartialRoom room;
+        room.tail = W + (size_t) group * img;
+        room.tail_bytes = workspace_bytes - (kHeaderBytes + tb +
+                (size_t) group * img);
+        if ((err = launch_gemm(gp, s, room))) return err;
         if (after_group) after_group(ctx, p0, np);
     }
     return 0;
@@ -3876,7 +4185,7 @@ extern "C" int oskb_cross_correlate_tc_noalloc_d(int casa, int num_sources,
     return jones_block(casa, num_sources, num_stations, offset_out, jones, I,
             Q, U, V, station_u, station_v, uv_min_lambda, uv_max_lambda,
             inv_wavelength, vis, reinterpret_cast<uint8_t*>(scratch),
-            as_stream(stream));
+            as_stream(stream), false);
 }
 
 // Status words of the last allocation-free call on the current device: the
