@@ -3091,6 +3091,29 @@ int get_workspace(void*& ws, size_t& ws_bytes, size_t need,
     return 0;
 }
 
+// Images of a library-kept workspace: a group of at most max_group() problems
+// (fixed bytes: header and tables) of `img` bytes each. A kept workspace that
+// holds the group is used as it is; only one that has to grow asks the driver
+// for the free memory (which costs tens of microseconds) and takes at most
+// half of it.
+int kept_group(int num_problems, size_t fixed, size_t img,
+        cudaStream_t stream)
+{
+    const int most = std::min(num_problems, max_group());
+    const int dev = current_device();
+    {
+        std::lock_guard<std::mutex> lock(g_ws_mutex);
+        for (const auto& w : g_ws)
+            if (w.dev == dev && w.stream == stream &&
+                    w.bytes >= fixed + (size_t) most * img)
+                return most;
+    }
+    size_t free_b = 0, total_b = 0;
+    cudaMemGetInfo(&free_b, &total_b);
+    const size_t fit = std::max<size_t>(1, free_b / 2 / img);
+    return (int) std::min<size_t>(fit, (size_t) most);
+}
+
 // Optional CUDA-event timing of every GEMM launch (for roofline reports),
 // guarded by a lock so that launches from several host threads are all
 // recorded.
@@ -3648,12 +3671,7 @@ int correlate_block_l6(int casa, int num_sources, int num_stations,
     }
     else
     {
-        size_t free_b = 0, total_b = 0;
-        cudaMemGetInfo(&free_b, &total_b);
-        size_t fit = free_b / 2 / img;
-        if (fit < 1) fit = 1;
-        if ((size_t) group > fit) group = (int) fit;
-        if (group > max_group()) group = max_group();
+        group = kept_group(num_problems, kHeaderBytes + tb, img, s);
     }
     int err = get_workspace(workspace, workspace_bytes,
             kHeaderBytes + tb + (size_t) group * img, s);
@@ -3957,12 +3975,8 @@ int correlate_block(int casa, int num_sources, int num_stations,
     {
         // Library-kept workspace: at most max_group() images, and no more
         // than half of the device memory that is free now.
-        size_t free_b = 0, total_b = 0;
-        cudaMemGetInfo(&free_b, &total_b);
-        size_t fit = free_b / 2 / img;
-        if (fit < 1) fit = 1;
-        if ((size_t) group > fit) group = (int) fit;
-        if (group > max_group()) group = max_group();
+        group = kept_group(num_problems, kHeaderBytes + tb, img,
+                as_stream(stream));
     }
     cudaStream_t s = as_stream(stream);
     int err = get_workspace(workspace, workspace_bytes,
