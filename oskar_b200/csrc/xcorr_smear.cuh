@@ -91,6 +91,7 @@ struct SmearSmem
     // x, y pair (time smearing).
     T st_uvw[2][kTile][3];
     double st_xy[2][kTile][2];
+    unsigned bound[2];   // longest baseline of the tile in phase units (bits)
 };
 
 // sinc(d) = sin(d) / d of a phase difference d, from the per-station sin and
@@ -105,15 +106,33 @@ struct SmearSmem
 // (FP32). Both forms are evaluated and one selected (no divergence within a
 // warp), as a numerator and a denominator (sin d, d) or (series, 1), so that
 // the bandwidth and time factors of a source-baseline share one reciprocal.
-__device__ __forceinline__ void sinc_parts(double d, double by_identity,
-        double& num, double& den)
+template <typename T>
+constexpr T kSincTau = sizeof(T) == 8 ? (T) (1.0 / 16) : (T) 0.5;
+
+__device__ __forceinline__ double sinc_series(double d)
 {
     constexpr double t = 1.0 / 256, c4 = 1.0 / 362880;
     constexpr double a3 = -1.0 / 5040 + c4 * 2 * t;
     constexpr double a2 = 1.0 / 120 - c4 * 1.25 * t * t;
     constexpr double a1 = -1.0 / 6 + c4 * 0.25 * t * t * t;
     const double y = d * d;
-    const double by_series = fma(y, fma(y, fma(y, a3, a2), a1), 1.0);
+    return fma(y, fma(y, fma(y, a3, a2), a1), 1.0);
+}
+
+__device__ __forceinline__ f32x2 sinc_series(f32x2 d)
+{
+    const f32x2 y = mul2(d, d);
+    f32x2 s = fma2(y, pack2((float) (1.0 / 362880), (float) (1.0 / 362880)),
+            pack2((float) (-1.0 / 5040), (float) (-1.0 / 5040)));
+    s = fma2(y, s, pack2((float) (1.0 / 120), (float) (1.0 / 120)));
+    s = fma2(y, s, pack2((float) (-1.0 / 6), (float) (-1.0 / 6)));
+    return fma2(y, s, pack2(1.0f, 1.0f));
+}
+
+__device__ __forceinline__ void sinc_parts(double d, double by_identity,
+        double& num, double& den)
+{
+    const double by_series = sinc_series(d);
     // |d| < 1/16 by its exponent (an integer comparison; false for NaN)
     const bool small = (__double2hiint(d) & 0x7fffffff) < 0x3fb00000;
     num = small ? by_series : by_identity;
@@ -193,6 +212,26 @@ __device__ __forceinline__ void smear_issue_src(SmearSmem<T, MATRIX>& sm,
     cp_async_commit();
 }
 
+// The larger value, or NaN where one is (as bits of a non-negative value).
+__device__ __forceinline__ float max_or_nan(float a, float b)
+{
+    return __uint_as_float(max(__float_as_uint(a), __float_as_uint(b)));
+}
+
+// Whether every phase difference of a chunk is below tau: reach is the
+// chunk's largest |(l, m, n - 1)|, bw and ts the longest baseline in phase
+// units (0 without that smearing). False for NaN. The series alone is taken
+// in FP32 only, where tau = 1/2 covers arrays of a few km (125 stations x
+// 7,000 sources, 3 km: 2.6 times the four-baseline kernel, 1.6 without); in
+// FP64 tau = 1/16 seldom holds, and the second loop cost 3 to 5 % where it
+// did not.
+template <typename T>
+__device__ __forceinline__ bool sinc_small(float reach, float bw, float ts)
+{
+    return sizeof(T) == 4 && reach * bw < (float) kSincTau<T> &&
+            reach * ts < (float) kSincTau<T>;
+}
+
 // Stores one element's factor values.
 template <int NC>
 __device__ __forceinline__ void put_entry(SmearFactors<double, NC>& f,
@@ -217,19 +256,22 @@ __device__ __forceinline__ void put_entry(SmearFactors<float, NC>& f,
 }
 template <int NC>
 __device__ __forceinline__ void put_phase(SmearFactors<double, NC>& f,
-        int which, int blk, int sl, int stl, double ph, const double2* trig)
+        int which, int blk, int sl, int stl, double ph, const double2* trig,
+        bool small)
 {
+    f.phi[which][blk][sl][stl] = ph;
+    if (small) return;
     double sn, cs;
     trig_steps_checked(trig, ph * kTrigStepsPerRadian, &sn, &cs);
-    f.phi[which][blk][sl][stl] = ph;
     f.sc[which][blk][sl][stl] = make_double2(sn, cs);
 }
 template <int NC>
 __device__ __forceinline__ void put_phase(SmearFactors<float, NC>& f,
-        int which, int blk, int sl, int stl, float ph, const double2*)
+        int which, int blk, int sl, int stl, float ph, const double2*,
+        bool small)
 {
-    float sn, cs;
-    sincosf(ph, &sn, &cs);
+    float sn = 0.0f, cs = 1.0f;
+    if (!small) sincosf(ph, &sn, &cs);
     if (blk)
     {
         float* o = &f.col_ps[which][sl][stl >> 1].x + (stl & 1);
@@ -251,7 +293,7 @@ template <typename T, bool MATRIX, bool GAUSS, bool BW, bool TS, bool CASA,
         bool FUSED>
 __device__ __forceinline__ void smear_transform(SmearSmem<T, MATRIX>& sm,
         const XcorrParams<T>& prm, bool have_jones, const ItemCtx& ctx,
-        T wavenumber, bool in_range, int buf)
+        T wavenumber, bool in_range, int buf, float& reach)
 {
     typedef typename vec2<T>::type T2;
     typedef Staging<T, MATRIX> G;
@@ -353,20 +395,35 @@ __device__ __forceinline__ void smear_transform(SmearSmem<T, MATRIX>& sm,
         const double* xy = sm.st_xy[blk][stl];
         const double l = src[kL][sl], m = src[kM][sl];
         const double n1 = (double) src[kN][sl] - 1.0;
+        // the chunk's largest |(l, m, n - 1)|: times a baseline's length in
+        // phase units, it bounds the phase differences of the chunk (for
+        // the time smearing too: (s m - c (n - 1)) is no longer than
+        // (m, n - 1))
+        if (sizeof(T) == 4)
+        {
+            const float r = in_range ? 1.0001f * sqrtf((float) (l * l +
+                    m * m + n1 * n1)) : 0.0f;
+            reach = __uint_as_float(__reduce_max_sync(0xffffffffu,
+                    __float_as_uint(r)));
+        }
+        const bool small = sinc_small<T>(reach, __uint_as_float(sm.bound[0]),
+                __uint_as_float(sm.bound[1]));
         if (BW)
             put_phase(f, 0, blk, sl, stl, (T) (((double) u[0] * l +
                     (double) u[1] * m + (double) u[2] * n1) * prm.bw_scale),
-                    sm.trig);
+                    sm.trig, small);
         if (TS)
             put_phase(f, 1, blk, sl, stl, (T) ((xy[0] * l + xy[1] *
-                    (prm.s_dec * m - prm.c_dec * n1)) * ctx.ts_scale), sm.trig);
+                    (prm.s_dec * m - prm.c_dec * n1)) * ctx.ts_scale), sm.trig,
+                    small);
     }
     if (GAUSS && warp < 3 && lane < kChunk)
         f.gauss[lane][warp] = src[kGa + warp][lane];
 }
 
 // One chunk's products, FP64: the thread's rows pr, pr + 1 and column qc.
-template <bool MATRIX, bool GAUSS, bool BW, bool TS, bool CASA>
+// SMALL: every phase difference of the warp's patch is below tau.
+template <bool MATRIX, bool GAUSS, bool BW, bool TS, bool CASA, bool SMALL>
 __device__ __forceinline__ void smear_products(
         const SmearFactors<double, MATRIX ? 4 : 1>& f, int ns, int pr, int qc,
         const double (&uu2)[2], const double (&vv2)[2],
@@ -378,7 +435,22 @@ __device__ __forceinline__ void smear_products(
     {
         // ---- factors of the two baselines
         double w[2] = {1.0, 1.0};
-        if (BW || TS)
+        if ((BW || TS) && SMALL)
+        {
+#pragma unroll
+            for (int which = BW ? 0 : 1; which < (TS ? 2 : 1); ++which)
+            {
+                const double pb = f.phi[which][1][sl][qc];
+#pragma unroll
+                for (int i = 0; i < 2; ++i)
+                {
+                    const double x = sinc_series(
+                            f.phi[which][0][sl][pr + i] - pb);
+                    w[i] = BW && which == 1 ? w[i] * x : x;
+                }
+            }
+        }
+        else if (BW || TS)
         {
             double num[2], den[2];
 #pragma unroll
@@ -413,7 +485,7 @@ __device__ __forceinline__ void smear_products(
                     w[i] *= exp(-(ga * uu2[i] + gb * uuvv[i] + gc * vv2[i]));
             }
         }
-        // ---- products, the factor applied to the row's values
+        // ---- products: each part of L R^H, then times the factor
         double2 C[NC];
 #pragma unroll
         for (int k = 0; k < NC; ++k) C[k] = f.col[k][sl][qc];
@@ -422,35 +494,27 @@ __device__ __forceinline__ void smear_products(
         {
             double2 R[NC];
 #pragma unroll
-            for (int k = 0; k < NC; ++k)
-            {
-                R[k] = f.row[k][sl][pr + i];
-                R[k].x *= w[i];
-                R[k].y *= w[i];
-            }
+            for (int k = 0; k < NC; ++k) R[k] = f.row[k][sl][pr + i];
             const double2* L = CASA ? C : R;
             const double2* Rt = CASA ? R : C;
             double* o = acc[i];
 #pragma unroll
-            for (int u = 0; u < (MATRIX ? 2 : 1); ++u)
+            for (int e = 0; e < NC; ++e)
             {
+                // element e = (r, c): sum_u L[2r + u] conj(Rt[2c + u])
+                double re = 0, im = 0;
 #pragma unroll
-                for (int e = 0; e < NC; ++e)
-                {
-                    // element e = (r, c): sum_u L[2r + u] conj(Rt[2c + u])
-                    const double2 x = L[MATRIX ? 2 * (e >> 1) + u : 0];
-                    const double2 y = Rt[MATRIX ? 2 * (e & 1) + u : 0];
-                    o[2 * e] = fma(x.x, y.x, o[2 * e]);
-                    o[2 * e + 1] = fma(x.y, y.x, o[2 * e + 1]);
-                }
-#pragma unroll
-                for (int e = 0; e < NC; ++e)
+                for (int u = 0; u < (MATRIX ? 2 : 1); ++u)
                 {
                     const double2 x = L[MATRIX ? 2 * (e >> 1) + u : 0];
                     const double2 y = Rt[MATRIX ? 2 * (e & 1) + u : 0];
-                    o[2 * e] = fma(x.y, y.y, o[2 * e]);
-                    o[2 * e + 1] = fma(-x.x, y.y, o[2 * e + 1]);
+                    re = u ? fma(x.x, y.x, re) : x.x * y.x;
+                    im = u ? fma(x.y, y.x, im) : x.y * y.x;
+                    re = fma(x.y, y.y, re);
+                    im = fma(-x.x, y.y, im);
                 }
+                o[2 * e] = fma(re, w[i], o[2 * e]);
+                o[2 * e + 1] = fma(im, w[i], o[2 * e + 1]);
             }
         }
     }
@@ -458,7 +522,7 @@ __device__ __forceinline__ void smear_products(
 
 // One chunk's products, FP32: the thread's row pr and columns qc, qc + 1 as
 // packed pairs; the chunk's sums are added to the FP64 sums at its end.
-template <bool MATRIX, bool GAUSS, bool BW, bool TS, bool CASA>
+template <bool MATRIX, bool GAUSS, bool BW, bool TS, bool CASA, bool SMALL>
 __device__ __forceinline__ void smear_products(
         const SmearFactors<float, MATRIX ? 4 : 1>& f, int ns, int pr, int qc,
         const float (&uu2)[2], const float (&vv2)[2],
@@ -473,7 +537,22 @@ __device__ __forceinline__ void smear_products(
     for (int sl = 0; sl < ns; ++sl)
     {
         float w[2] = {1.0f, 1.0f};
-        if (BW || TS)
+        if ((BW || TS) && SMALL)
+        {
+            f32x2 x = 0;
+#pragma unroll
+            for (int which = BW ? 0 : 1; which < (TS ? 2 : 1); ++which)
+            {
+                const f32x2 a = *reinterpret_cast<const f32x2*>(
+                        &f.row_ps[which][sl][pr]);
+                const f32x2 b = *reinterpret_cast<const f32x2*>(
+                        &f.col_ps[which][sl][qp]);
+                const f32x2 y = sinc_series(fma2(b, pack2(-1.0f, -1.0f), a));
+                x = BW && which == 1 ? mul2(x, y) : y;
+            }
+            unpack2(x, w[0], w[1]);
+        }
+        else if (BW || TS)
         {
             float num[2], den[2];
 #pragma unroll
@@ -489,15 +568,7 @@ __device__ __forceinline__ void smear_products(
                         &f.col_c[which][sl][qp]);
                 const f32x2 d = fma2(b.x, pack2(-1.0f, -1.0f), a.x);
                 const f32x2 ident = fma2(nca, b.y, mul2(a.y, cb));
-                const f32x2 d2 = mul2(d, d);
-                f32x2 ser = fma2(d2, pack2((float) (1.0 / 362880),
-                        (float) (1.0 / 362880)), pack2((float) (-1.0 / 5040),
-                        (float) (-1.0 / 5040)));
-                ser = fma2(d2, ser, pack2((float) (1.0 / 120),
-                        (float) (1.0 / 120)));
-                ser = fma2(d2, ser, pack2((float) (-1.0 / 6),
-                        (float) (-1.0 / 6)));
-                ser = fma2(d2, ser, pack2(1.0f, 1.0f));
+                const f32x2 ser = sinc_series(d);
                 float dd[2], id[2], se[2];
                 unpack2(d, dd[0], dd[1]);
                 unpack2(ident, id[0], id[1]);
@@ -505,7 +576,7 @@ __device__ __forceinline__ void smear_products(
 #pragma unroll
                 for (int j = 0; j < 2; ++j)
                 {
-                    const bool small = fabsf(dd[j]) < 0.5f;
+                    const bool small = fabsf(dd[j]) < kSincTau<float>;
                     const float nu = small ? se[j] : id[j];
                     const float de = small ? 1.0f : dd[j];
                     const bool first = !(BW && which == 1);
@@ -531,21 +602,15 @@ __device__ __forceinline__ void smear_products(
             }
         }
         const f32x2 ww = pack2(w[0], w[1]);
-        // the factors applied to the column pair's values; real and
-        // imaginary parts as packed pairs
-        f32x2 cr[NC], ci[NC];
+        // real and imaginary parts of the column pair and the row
+        f32x2 cr[NC], ci[NC], rr[NC], ri[NC];
 #pragma unroll
         for (int k = 0; k < NC; ++k)
         {
             const ulonglong2 c = *reinterpret_cast<const ulonglong2*>(
                     &f.col[k][sl][qp]);
-            cr[k] = mul2(c.x, ww);
-            ci[k] = mul2(c.y, ww);
-        }
-        f32x2 rr[NC], ri[NC];
-#pragma unroll
-        for (int k = 0; k < NC; ++k)
-        {
+            cr[k] = c.x;
+            ci[k] = c.y;
             const ulonglong2 r = *reinterpret_cast<const ulonglong2*>(
                     &f.row[k][sl][pr]);
             rr[k] = r.x;
@@ -560,24 +625,21 @@ __device__ __forceinline__ void smear_products(
 #pragma unroll
         for (int k = 0; k < NC; ++k) nyi[k] = neg2(yi[k]);
 #pragma unroll
-        for (int u = 0; u < (MATRIX ? 2 : 1); ++u)
+        for (int e = 0; e < NC; ++e)
         {
+            f32x2 re = 0, im = 0;
 #pragma unroll
-            for (int e = 0; e < NC; ++e)
+            for (int u = 0; u < (MATRIX ? 2 : 1); ++u)
             {
                 const int x = MATRIX ? 2 * (e >> 1) + u : 0;
                 const int y = MATRIX ? 2 * (e & 1) + u : 0;
-                part[2 * e] = fma2(xr[x], yr[y], part[2 * e]);
-                part[2 * e + 1] = fma2(xi[x], yr[y], part[2 * e + 1]);
+                re = u ? fma2(xr[x], yr[y], re) : mul2(xr[x], yr[y]);
+                im = u ? fma2(xi[x], yr[y], im) : mul2(xi[x], yr[y]);
+                re = fma2(xi[x], yi[y], re);
+                im = fma2(xr[x], nyi[y], im);
             }
-#pragma unroll
-            for (int e = 0; e < NC; ++e)
-            {
-                const int x = MATRIX ? 2 * (e >> 1) + u : 0;
-                const int y = MATRIX ? 2 * (e & 1) + u : 0;
-                part[2 * e] = fma2(xi[x], yi[y], part[2 * e]);
-                part[2 * e + 1] = fma2(xr[x], nyi[y], part[2 * e + 1]);
-            }
+            part[2 * e] = fma2(re, ww, part[2 * e]);
+            part[2 * e + 1] = fma2(im, ww, part[2 * e + 1]);
         }
     }
 #pragma unroll
@@ -628,6 +690,7 @@ xcorr_smear_kernel(const XcorrParams<T> prm)
             (ctx.src_end - ctx.src_begin + kChunk - 1) / kChunk : 0;
 
     __syncthreads();  // the previous item is done with shared memory
+    if (tid < 2) sm.bound[tid] = 0;
     if (nchunks > 0)
     {
         if (warp == kSrcWarp)
@@ -663,6 +726,7 @@ xcorr_smear_kernel(const XcorrParams<T> prm)
     const T uv_lo = (T) (prm.uv_min * uv_scale);
     const T uv_hi = (T) (prm.uv_max * uv_scale);
     bool exists[2], valid[2];
+    float longest[2] = {0.0f, 0.0f};   // baselines in phase units: bw, ts
     T uu2[2], vv2[2], uuvv[2];
 #pragma unroll
     for (int i = 0; i < 2; ++i)
@@ -678,6 +742,20 @@ xcorr_smear_kernel(const XcorrParams<T> prm)
             vv = (sv[p] - sv[q]) * (T) ctx.inv_wavelength;
             const T len = sqrt(uu * uu + vv * vv);
             ok = !(len < uv_lo || len > uv_hi);
+            if (BW && !F64)
+            {
+                const double du = su[p] - su[q], dv = sv[p] - sv[q],
+                        dw = sw[p] - sw[q];
+                longest[0] = max_or_nan(longest[0], (float) (fabs(
+                        prm.bw_scale) * sqrt(du * du + dv * dv + dw * dw)));
+            }
+            if (TS && !F64)
+            {
+                const double dx = prm.st_x[p] - prm.st_x[q],
+                        dy = prm.st_y[p] - prm.st_y[q];
+                longest[1] = max_or_nan(longest[1], (float) (fabs(
+                        ctx.ts_scale) * sqrt(dx * dx + dy * dy)));
+            }
         }
         valid[i] = ok;
         uu2[i] = uu * uu;
@@ -685,6 +763,13 @@ xcorr_smear_kernel(const XcorrParams<T> prm)
         uuvv[i] = 2 * uu * vv;
     }
     const bool active = __any_sync(0xffffffffu, valid[0] || valid[1]);
+    if ((BW || TS) && !F64)
+    {
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+            longest[k] = __uint_as_float(__reduce_max_sync(0xffffffffu,
+                    __float_as_uint(longest[k])));
+    }
 
     double acc[2][2 * NC];
 #pragma unroll
@@ -693,18 +778,20 @@ xcorr_smear_kernel(const XcorrParams<T> prm)
         for (int k = 0; k < 2 * NC; ++k) acc[i][k] = 0.0;
 
     // Transform of chunk c into buffer c & 1, then the copies of chunk
-    // c + 1 into the warp's raw buffer.
+    // c + 1 into the warp's raw buffer. Returns the chunk's reach.
     const auto advance = [&](int c)
     {
+        float reach = 0.0f;
         const int s0 = ctx.src_begin + c * kChunk;
         cp_async_wait_all();
         __syncwarp();   // the warp's own copies, visible to its lanes
         smear_transform<T, MATRIX, GAUSS, BW, TS, CASA, FUSED>(sm, prm,
                 jsrc != nullptr, ctx, wavenumber, s0 + (lane & 7) <
-                ctx.src_end, c & 1);
+                ctx.src_end, c & 1, reach);
         __syncwarp();
         if (c + 1 < nchunks)
             smear_issue<T, MATRIX>(sm, prm, jsrc, ctx, s0 + kChunk);
+        return reach;
     };
     // The per-source values of chunk c + 1, in buffer (c + 1) & 1, are read
     // by chunk c's iteration: copied one iteration earlier by one warp, whose
@@ -717,10 +804,17 @@ xcorr_smear_kernel(const XcorrParams<T> prm)
     };
     cp_async_wait_all();
     __syncthreads();  // per-station terms and chunk 0's values are there
+    float reach = 0.0f, reach_next = 0.0f;
+    if ((BW || TS) && !F64)
+    {
+        if (lane < 2) atomicMax(&sm.bound[lane], __float_as_uint(
+                lane ? longest[1] : longest[0]));
+        __syncthreads();
+    }
     if (nchunks > 0)
     {
         issue_src(1);
-        advance(0);
+        reach = advance(0);
     }
     __syncthreads();
 #pragma unroll 1
@@ -733,14 +827,20 @@ xcorr_smear_kernel(const XcorrParams<T> prm)
         {
             if ((step == 0) == early)
             {
-                if (c + 1 < nchunks) advance(c + 1);
+                if (c + 1 < nchunks) reach_next = advance(c + 1);
             }
             else if (active)
             {
-                smear_products<MATRIX, GAUSS, BW, TS, CASA>(sm.f[c & 1], ns,
-                        pr, qc, uu2, vv2, uuvv, acc);
+                if ((BW || TS) && sinc_small<T>(reach, longest[0],
+                        longest[1]))
+                    smear_products<MATRIX, GAUSS, BW, TS, CASA, true>(
+                            sm.f[c & 1], ns, pr, qc, uu2, vv2, uuvv, acc);
+                else
+                    smear_products<MATRIX, GAUSS, BW, TS, CASA, false>(
+                            sm.f[c & 1], ns, pr, qc, uu2, vv2, uuvv, acc);
             }
         }
+        reach = reach_next;
         __syncthreads();  // chunk c consumed, chunk c + 1's factors ready
     }
 

@@ -36,3 +36,22 @@ def test_patches_chunks_and_mixed_sources(num_st, num_src, real, matrix, bw,
     for k in "abc":
         getattr(c, k)[point] = 0
     assert_close(run_gpu_xcorr(c, real), run_oracle_xcorr(c, real), real)
+
+
+@pytest.mark.parametrize("real", [np.float64, np.float32])
+@pytest.mark.parametrize("bw,ts", [(100e3, 0.0), (0.0, 10.0), (100e3, 10.0)])
+@pytest.mark.parametrize("core", [0, 8, 20, 70])
+def test_short_and_long_baselines(real, bw, ts, core):
+    """Patches whose phase differences are all small take the series alone,
+    the others the identity too: a core of stations within 60 m (FP64) or
+    400 m (FP32) and the rest up to 60 (6) km, from none of one to none of
+    the other. FP32 phases of 0.02 x 6 km carry 120 x 6e-8 absolute error:
+    1e-5 as above."""
+    c = XcorrCase(70, 57, real=real, ranges="physical", bandwidth_hz=bw,
+                  time_avg=ts, gaussian=False, seed=core + 1)
+    near, far = (0.06, 60.0) if real == np.float64 else (0.4, 6.0)
+    scale = np.where(np.arange(70) < core, near, far).astype(real)
+    for k in ("st_u", "st_v", "st_w", "st_x", "st_y"):
+        setattr(c, k, (getattr(c, k) * scale * real(2 if k[-1] in "uvw"
+                                                    else 1)).astype(real))
+    assert_close(run_gpu_xcorr(c, real), run_oracle_xcorr(c, real), real)
