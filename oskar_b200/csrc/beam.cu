@@ -303,7 +303,7 @@ __device__ __forceinline__ void station_beam_item(BeamSmem<T, IS3D, NT>& sm,
     const TypeParams<T>& tp = arg.tp;
     const double* beam_enu = arg.beam_enu;
     const int rows = arg.rows;
-    const int d0 = d_first + threadIdx.x;
+    const int d0 = d_first + threadIdx.x, threads = blockDim.x;
     const size_t el0 = (size_t) st * num_elements;
     const size_t dir0 = arg.directions_per_station ? (size_t) st * num_dir : 0;
     const int per_dir = flags.scalar ? 1 : 4;
@@ -316,7 +316,7 @@ __device__ __forceinline__ void station_beam_item(BeamSmem<T, IS3D, NT>& sm,
 #pragma unroll
         for (int j = 0; j < ND; ++j)
         {
-            const int d = d0 + j * kThreads;
+            const int d = d0 + j * threads;
             if (d < num_dir)
                 for (int k = 0; k < per_dir; ++k)
                     out[(size_t) per_dir * d + k] = T2{(T) 0, (T) 0};
@@ -337,7 +337,7 @@ __device__ __forceinline__ void station_beam_item(BeamSmem<T, IS3D, NT>& sm,
 #pragma unroll
     for (int j = 0; j < ND; ++j)
     {
-        const int d = d0 + j * kThreads;
+        const int d = d0 + j * threads;
         X[j] = Y[j] = Z[j] = 0;
         if (d < num_dir)
         {
@@ -389,7 +389,7 @@ __device__ __forceinline__ void station_beam_item(BeamSmem<T, IS3D, NT>& sm,
         }
         __syncthreads();
         unsigned ex = 0, ey = 0, ez = 0;
-        for (int t = threadIdx.x; t < ne; t += kThreads)
+        for (int t = threadIdx.x; t < ne; t += threads)
         {
             const size_t g = el0 + e0 + t;
             const T x = arg.el_x[g], y = arg.el_y[g], z = arg.el_z ? arg.el_z[g] : (T) 0;
@@ -526,7 +526,7 @@ __device__ __forceinline__ void station_beam_item(BeamSmem<T, IS3D, NT>& sm,
         for (int t = 0; t < NT; ++t)
         {
             nr[t] = ni[t] = 0;
-            for (int w = 0; w < kThreads / 32; ++w)
+            for (int w = 0; w < threads / 32; ++w)
             {
                 nr[t] += sm.red[0][t][w];
                 ni[t] += sm.red[1][t][w];
@@ -606,7 +606,7 @@ __device__ __forceinline__ void station_beam_item(BeamSmem<T, IS3D, NT>& sm,
 #pragma unroll 1
     for (int j = 0; j < ND; ++j)
     {
-        const int d = d0 + j * kThreads;
+        const int d = d0 + j * threads;
         if (d >= num_dir) break;
         T2* o = out + (size_t) per_dir * d;
         T x = X[0], y = Y[0], z = Z[0], fr[NT], fi[NT];
@@ -684,8 +684,8 @@ __device__ __forceinline__ void station_beam_item(BeamSmem<T, IS3D, NT>& sm,
 }
 
 // One CTA takes items in turn, with its table filled once: first `full`
-// (station, block of kThreads x BIG directions) items in whole rounds of the
-// grid, then the rest in quarters or halves of kThreads x SMALL directions,
+// (station, block of threads x BIG directions) items in whole rounds of the
+// grid, then the rest in quarters or halves of threads x SMALL directions,
 // so that the last round is short: at 128 stations x 12,000 directions a
 // grid of 296 has 5.2 rounds of 1,024 directions, and a whole sixth round
 // would idle most of the chip. More directions per thread share the staged
@@ -702,14 +702,15 @@ station_beam_kernel(const __grid_constant__ BeamArgs<T> arg, int blocks,
     Trig<T>::fill(sm.table);
     for (int item = blockIdx.x; item < full; item += gridDim.x)
         station_beam_item<T, IS3D, NT, BIG>(sm, arg, item / blocks,
-                item % blocks * (kThreads * BIG));
-    constexpr int PARTS = BIG / SMALL;
-    for (int part = blockIdx.x; part < (items - full) * PARTS;
-            part += gridDim.x)
+                item % blocks * ((int) blockDim.x * BIG));
+    // the rest part by part, so that the empty ones past the last direction
+    // come last
+    const int rest = items - full;
+    for (int n = blockIdx.x; n < rest * (BIG / SMALL); n += gridDim.x)
     {
-        const int item = full + part / PARTS;
-        const int d = (item % blocks * PARTS + part % PARTS) *
-                (kThreads * SMALL);
+        const int item = full + n % rest, part = n / rest;
+        const int d = item % blocks * ((int) blockDim.x * BIG) + part *
+                ((int) blockDim.x * SMALL);
         if (d < arg.num_dir)
             station_beam_item<T, IS3D, NT, SMALL>(sm, arg, item / blocks, d);
     }
@@ -875,14 +876,30 @@ int station_beam_aa(int num_stations, int num_elements, const T* el_x,
     const double wavenumber = 2.0 * kPi * frequency_hz / c0;
     BeamFlags flags{normalise_element, normalise_array, normalise_final,
             swap_xy, scalar};
+    // Threads per CTA: fewer where blocks of 256 x kDirsSmall directions do
+    // not give every SM one (1 station x 20,000 directions: 79 of them) or
+    // would be half empty; an SM then takes more CTAs (two tables of 64 KB or
+    // four of 32 fit).
+    const int sms = device_sm_count();
+    constexpr int small = kDirsSmall<T>;
+    int threads = kThreads;
+    while (threads > 64 && (num_directions <= threads / 2 * small ||
+            ((long long) num_directions + threads * small - 1) /
+            (threads * small) * num_stations < sms))
+        threads /= 2;
+    const int per_sm = std::min(sizeof(T) == 8 ? kCtasPerSm : 2 * kCtasPerSm,
+            kCtasPerSm * kThreads / threads);
     const int big = dirs_big<T>(num_element_types);
     const int parts = big / kDirsSmall<T>;
-    const int blocks = (int) (((long long) num_directions + kThreads * big -
-            1) / (kThreads * big));
+    const int blocks = (int) (((long long) num_directions + threads * big -
+            1) / (threads * big));
     const long long items = (long long) blocks * num_stations;
     if (items > INT_MAX / parts) return OSKB_ERR_INVALID_ARGUMENT;
-    const int slots = kCtasPerSm * device_sm_count();
-    const int full = (int) (items / slots * slots);
+    const int slots = per_sm * sms;
+    // whole rounds of big items, unless their blocks would be a quarter
+    // empty or more
+    const bool dense = 4LL * num_directions >= 3LL * blocks * threads * big;
+    const int full = dense ? (int) (items / slots * slots) : 0;
     const int grid = full ? slots : (int) std::min<long long>(slots, items *
             parts);
     const BeamArgs<T> arg = {num_elements, el_x, el_y, el_z, meas_x, meas_y,
@@ -898,7 +915,7 @@ int station_beam_aa(int num_stations, int num_elements, const T* el_x,
         const int smem = (int) sizeof(BeamSmem<T, D, NT>);                   \
         cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, \
                 smem);                                                       \
-        k<<<grid, kThreads, smem, s>>>(arg, blocks, (int) items, full);      \
+        k<<<grid, threads, smem, s>>>(arg, blocks, (int) items, full);       \
     }
 #define OSKB_BEAM_NT(D)                                                      \
     switch (num_element_types)                                               \

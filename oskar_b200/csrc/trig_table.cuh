@@ -49,9 +49,11 @@ __device__ __forceinline__ void trig_table_fill(double2* table)
     {
         double s, c;
         sincospi((double) j / (kTrigEntries / 2), &s, &c);
+        // (each lane starts at its own copy: distinct banks)
 #pragma unroll
         for (int k = 0; k < kTrigCopies; ++k)
-            table[j * kTrigCopies + k] = make_double2(c, s);
+            table[j * kTrigCopies + ((k + j) & (kTrigCopies - 1))] =
+                    make_double2(c, s);
     }
 }
 
@@ -130,9 +132,11 @@ template <> struct Trig<double>
         {
             double s, c;
             sincospi((double) j / (kEntries / 2), &s, &c);
+            // (each lane starts at its own copy: distinct banks)
 #pragma unroll
             for (int k = 0; k < kCopies; ++k)
-                table[j * kCopies + k] = make_double2(c, s);
+                table[j * kCopies + ((k + j) & (kCopies - 1))] =
+                        make_double2(c, s);
         }
     }
     static __device__ __forceinline__ void sincos(const Entry* table,
@@ -185,7 +189,8 @@ template <> struct Trig<float>
             sincospif((float) j / (kEntries / 2), &s, &c);
 #pragma unroll
             for (int k = 0; k < kCopies; ++k)
-                table[j * kCopies + k] = make_float2(c, s);
+                table[j * kCopies + ((k + j) & (kCopies - 1))] =
+                        make_float2(c, s);
         }
     }
     // Two phases as a packed pair.
