@@ -192,8 +192,8 @@ OSKB_API int oskb_dftw_f(int matrix, int num_in, float wavenumber,
         int offset_out, float* output, float norm_factor, void* stream);
 
 /* out[2 i], out[2 i + 1] = cos, sin of (pi / 64) steps[i]: a phase given
- * in steps of 2 pi / 128, by the table-driven method the FP64 element loops
- * of the weighted DFT and the station beam use (128-entry table, Taylor
+ * in steps of 2 pi / 128, by the table-driven method the FP64 loops of the
+ * weighted DFT and the smearing correlation use (128-entry table, Taylor
  * series of the remainder; sincospi(steps / 64) where the table does not
  * reach, beyond |steps| = 2^32). Device arrays. No OSKAR counterpart:
  * exposed so the method can be checked against exact values. */

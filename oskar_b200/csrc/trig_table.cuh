@@ -1,6 +1,7 @@
-// Table-driven phase factors e^{i ph} in FP64 for the element loops of the
-// station beam and the weighted DFT, where one sincos per element-direction
-// bounds the kernel on the FP64 pipe.
+// Table-driven phase factors e^{i ph} for the element loops of the station
+// beam (Trig<T>, below, with larger tables) and, in FP64, of the weighted DFT
+// and the smearing kernel's transform, where one sincos per phase bounds the
+// kernel on the FP64 pipe.
 //
 // Method: P. T. P. Tang's table-driven scheme ("Table-lookup algorithms for
 // elementary functions and their error analysis", ARITH 1991). The loops
