@@ -16,8 +16,8 @@ blocks read back from the two .vis files must agree to
 and station-beam sums formed in a different order of operations), cross-
 and auto-correlations alike. The committed fixtures
 tests/golden/c1_sim*.npz hold the reference's output for the C1 cases
-(made by tests/golden/make_golden.py from the same harness), so that
-comparison also runs where the reference library is not built.
+(made by tests/golden/make_golden.py from the same harness). Every case
+needs the reference library, whose driver calls the drop-in.
 
 The reference's CPU path was seen to crash now and then (SIGSEGV in
 oskar_sky_scale_flux_with_frequency after its horizon clip): its runs keep
@@ -122,9 +122,11 @@ def test_dropin_matches_reference_run(name, precision, tmp_path):
 
 @pytest.mark.parametrize("name", ["c1", "c1_stations"])
 def test_dropin_matches_golden(name, tmp_path):
-    """Against the committed reference output (no reference library
-    needed); the drop-in also runs its own horizon clip, which keeps every
+    """Against the committed reference output (no run of the reference's CPU
+    path, but its library is loaded beside the drop-in, whose caller its
+    driver is); the drop-in also runs its own horizon clip, which keeps every
     source of this field."""
+    need_ref()
     case = CASES[name]("double")
     case["horizon_clip"] = 1
     got = run_sim(case, tmp_path, "b200", dropin=True)
