@@ -851,7 +851,14 @@ OSKB_API int oskb_evaluate_jones_R_f(int num_sources, const float* ra_rad,
  * smearing; station_u/v are only used by the uv filter.
  * workspace: device scratch of at least
  * oskb_cross_correlate_tc_workspace_bytes() bytes, or NULL to let the library
- * keep one per device (allocated on first use, grown on demand). */
+ * keep one per device (allocated on first use, grown on demand).
+ * A contraction of few tiles splits the last ones over the sources; the
+ * partial sums (at most 96 KB per SM, 64 KB in the FP64-class form) go behind
+ * the images in a workspace that is larger than needed by that much, as the
+ * library's own and a block plan's are, else to memory from the library's
+ * pool, and where that is not to be had (a stream being captured) the tiles
+ * run whole: the same results to the last bit. This holds for every entry
+ * point below that takes a workspace. */
 OSKB_API size_t oskb_cross_correlate_tc_workspace_bytes(int num_sources,
         int num_stations);
 OSKB_API int oskb_cross_correlate_tc_d(int use_casa_phase_convention,
@@ -1253,6 +1260,9 @@ OSKB_API int oskb_tc_status(const void* workspace, int* flags,
  * has at least two per SM, else square). Integer form: 128 (128 x 128 per
  * CTA). */
 OSKB_API int oskb_tc_tile_columns(void);
+/* Runs that each tile of the last, incomplete wave of the last integer
+ * contraction launched was split into (1: whole), 0 before the first. */
+OSKB_API int oskb_tc_last_wave_runs(void);
 /* Arithmetic of the last tensor-core contraction launched, 0 before the
  * first: 8 for the default integer form (the sources ordered into
  * amplitude buckets, factor 2 apart, each with its own scale; each scaled

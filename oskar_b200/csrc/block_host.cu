@@ -297,7 +297,7 @@ int plan_correlate(oskb_TcPlan* p, int k, int form,
             sky, sky + ns, sky + 2 * ns, sky + 3 * ns, sky + 4 * ns,
             sky + 5 * ns, sky + 6 * ns, static_cast<const double*>(s.uvw),
             p->wl, p->uv_min, p->uv_max, static_cast<double*>(s.vis), p->ws,
-            p->ws_bytes, p->compute, after, ctx, nullptr, form);
+            p->ws_bytes, p->compute, after, ctx, nullptr, form, false);
 }
 
 // Times each candidate form on slot k's (uploaded) block and keeps the
@@ -464,6 +464,21 @@ oskb_TcPlan* oskb_tc_plan_create(int casa, int num_sources, int num_stations,
     if (group < 1) group = 1;
     p->ws_bytes = oskb_correlate_block_tc_workspace_bytes(num_sources,
             num_stations, (int) group);
+    // and room for the integer form's partial sums, so that its last wave is
+    // split in the graphs as in the tuning run (whole where there is none)
+    const size_t room = tc::block_room(num_sources, num_stations,
+            num_problems, (int) group);
+    const auto alloc_ws = [&]()
+    {
+        if (cudaMalloc(&p->ws, p->ws_bytes + room) == cudaSuccess)
+        {
+            p->ws_bytes += room;
+            return true;
+        }
+        cudaGetLastError();
+        p->ws = nullptr;
+        return room > 0 && cudaMalloc(&p->ws, p->ws_bytes) == cudaSuccess;
+    };
     bool ok = cudaStreamCreateWithFlags(&p->in, cudaStreamNonBlocking) ==
             cudaSuccess &&
             cudaStreamCreateWithFlags(&p->compute, cudaStreamNonBlocking) ==
@@ -474,7 +489,7 @@ oskb_TcPlan* oskb_tc_plan_create(int casa, int num_sources, int num_stations,
             cudaSuccess &&
             cudaMalloc((void**) &p->wl, sizeof(double) * num_channels) ==
             cudaSuccess &&
-            cudaMalloc(&p->ws, p->ws_bytes) == cudaSuccess;
+            alloc_ws();
     for (auto& s : p->slot)
         ok = ok && cudaMalloc(&s.E, p->e_bytes) == cudaSuccess &&
                 cudaMalloc(&s.uvw, p->uvw_bytes) == cudaSuccess &&

@@ -3023,6 +3023,74 @@ int drain_kblocks()
     return d;
 }
 
+// ---- split of the last wave (TaskWalk)
+struct IntegerForm
+{
+    void (*gemm)(GemmParams);
+    void (*fixup)(GemmParams);
+    size_t smem;
+    int sums;      // of a thread: the fixup's grid height
+    int words;     // of a partial slot per thread
+    double kb_us;  // microseconds of one k block of a task
+};
+
+IntegerForm integer_form(bool six)
+{
+    if (six)
+        return {gemm_l6_kernel, fixup_l6_kernel, gemm_l6_smem_bytes(), 8,
+                kL6PartialWords, 1.8};
+    return {gemm_i8_kernel, fixup_i8_kernel, gemm_i8_smem_bytes(), 16,
+            kI8PartialWords, 0.72};
+}
+
+long long integer_tasks(bool six, int nrb, int num_problems)
+{
+    return (long long) nrb * (nrb + 1) / (six ? 1 : 2) * num_problems;
+}
+
+// Runs that each task of the last wave is split into: as many as fill the
+// idle SMs, of at least four of the at most nkb k blocks each, when that
+// saves more than the ~15 us of the partial sums and the second launch.
+int last_wave_pieces(const IntegerForm& f, long long ntasks, int nkb)
+{
+    const int sms = num_sms(), rest = (int) (ntasks % sms);
+    const int pieces = rest > 0 ? std::max(1, std::min(sms / rest, nkb / 4))
+            : 1;
+    return (1.0 - 1.0 / pieces) * nkb * f.kb_us > 15.0 ? pieces : 1;
+}
+
+size_t last_wave_bytes(const IntegerForm& f, long long ntasks, int nkb)
+{
+    const int pieces = last_wave_pieces(f, ntasks, nkb);
+    return pieces > 1 ? (size_t) (ntasks % num_sms()) * pieces * f.words *
+            256 * sizeof(uint32_t) : 0;
+}
+
+// Room for the partial sums of num_problems problems in groups of `group`.
+size_t partial_room(bool six, int num_st, int num_src, int num_problems,
+        int group)
+{
+    const IntegerForm f = integer_form(six);
+    const int nrb = (num_st + kStPerBlock - 1) / kStPerBlock;
+    const int cap = i8_kb_cap(num_src), last = num_problems % group;
+    return std::max(last_wave_bytes(f, integer_tasks(six, nrb,
+            std::min(group, num_problems)), cap), last_wave_bytes(f,
+            integer_tasks(six, nrb, last), cap));
+}
+
+// What lies behind the operand images: the tail of the workspace, and whether
+// the scratch pool may be used where that is too small.
+struct PartialRoom
+{
+    uint8_t* tail = nullptr;
+    size_t tail_bytes = 0;
+    bool pool = true;
+    PartialRoom() {}
+    PartialRoom(void* ws, size_t ws_bytes, size_t used, bool pool_ = true)
+            : tail(reinterpret_cast<uint8_t*>(ws) + used),
+              tail_bytes(ws_bytes - used), pool(pool_) {}
+};
+
 // Problems per group when the library keeps the workspace (each problem's
 // operand image is 32 bytes per station-source).
 int max_group()
@@ -3052,7 +3120,11 @@ std::mutex g_ws_mutex;
 std::vector<CachedWorkspace> g_ws;
 void* g_ws_last[64] = {};   // last library-kept workspace used per device
 
-int get_workspace(void*& ws, size_t& ws_bytes, size_t need,
+// The caller's workspace if it holds `need` bytes, else the library-kept one,
+// grown where it is smaller: to need + room bytes, or to need where that much
+// cannot be had. (A workspace that holds need is not grown for the room: work
+// recorded into a graph may use it.)
+int get_workspace(void*& ws, size_t& ws_bytes, size_t need, size_t room,
         cudaStream_t stream)
 {
     if (ws)
@@ -3077,13 +3149,19 @@ int get_workspace(void*& ws, size_t& ws_bytes, size_t need,
         }
         c->ptr = nullptr;
         c->bytes = 0;
-        if (cudaMalloc(&c->ptr, need) != cudaSuccess)
+        size_t get = need + room;
+        if (cudaMalloc(&c->ptr, get) != cudaSuccess)
         {
-            c->ptr = nullptr;
-            set_last_error("tc workspace", cudaGetLastError());
-            return OSKB_ERR_MEMORY_ALLOC_FAILURE;
+            cudaGetLastError();
+            get = need;
+            if (room == 0 || cudaMalloc(&c->ptr, get) != cudaSuccess)
+            {
+                c->ptr = nullptr;
+                set_last_error("tc workspace", cudaGetLastError());
+                return OSKB_ERR_MEMORY_ALLOC_FAILURE;
+            }
         }
-        c->bytes = need;
+        c->bytes = get;
     }
     ws = c->ptr;
     ws_bytes = c->bytes;
@@ -3134,6 +3212,7 @@ int tile_setting()
 }
 
 std::atomic<int> g_last_tile{0};
+std::atomic<int> g_last_pieces{0};
 std::atomic<int> g_last_arith{0};
 
 // Arithmetic of the contraction: the three-limb 8-bit integer form unless
@@ -3260,37 +3339,23 @@ cudaEvent_t timing_start(cudaStream_t stream)
     return g_ev[g_ev_used++].second;
 }
 
-// Room for the partial sums of a split last wave: the tail of the caller's
-// workspace where it is large enough, else the library's scratch pool (not
-// while the stream is captured, and not for the allocation-free entry
-// point), else none: the last wave's tasks then run whole, with the same
-// results to the last bit.
-struct PartialRoom
+// Launches an integer contraction: gemm, and fixup for a split last wave. The
+// partial sums go to the tail of the workspace where it has room, else to the
+// library's scratch pool (not while the stream is captured, not for a plan,
+// nor for the allocation-free entry point), else nowhere: the last wave's
+// tasks then run whole, with the same results to the last bit.
+int launch_integer(bool six, GemmParams& gp, const PartialRoom& room,
+        cudaStream_t stream)
 {
-    uint8_t* tail = nullptr;
-    size_t tail_bytes = 0;
-    bool pool = true;
-};
-
-// Launches an integer contraction (gemm, and fixup for a split last wave;
-// sums_per_thread: the fixup's grid height, words: of a partial slot per
-// thread) of ntasks tasks of at most nkb k blocks, kb_us microseconds each.
-// The last wave is split when that saves more than the ~15 us of the partial
-// sums and the second launch, into runs of at least four k blocks.
-int launch_integer(void (*gemm)(GemmParams), size_t smem,
-        void (*fixup)(GemmParams), int sums_per_thread, int words,
-        double kb_us, GemmParams& gp, long long ntasks,
-        const PartialRoom& room, cudaStream_t stream)
-{
+    const IntegerForm f = integer_form(six);
+    const long long ntasks = integer_tasks(six, gp.nrb, gp.num_problems);
     const int sms = num_sms();
-    const int rest = (int) (ntasks % sms);
     void* to_free = nullptr;
-    gp.pieces = rest > 0 ? std::max(1, std::min(sms / rest, gp.nkb / 4)) : 1;
+    gp.pieces = last_wave_pieces(f, ntasks, gp.nkb);
     gp.partial = nullptr;
-    if ((1.0 - 1.0 / gp.pieces) * gp.nkb * kb_us > 15.0)
+    if (gp.pieces > 1)
     {
-        const size_t need = (size_t) rest * gp.pieces * words * 256 *
-                sizeof(uint32_t);
+        const size_t need = last_wave_bytes(f, ntasks, gp.nkb);
         cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
         if (room.tail_bytes >= need)
             gp.partial = reinterpret_cast<uint32_t*>(room.tail);
@@ -3307,26 +3372,20 @@ int launch_integer(void (*gemm)(GemmParams), size_t smem,
         }
     }
     if (!gp.partial) gp.pieces = 1;
+    g_last_pieces.store(gp.pieces);
     const int grid = gp.partial || ntasks >= sms ? sms : (int) ntasks;
     cudaEvent_t ev_stop = timing_start(stream);
-    gemm<<<grid, kGemmThreads, smem, stream>>>(gp);
+    f.gemm<<<grid, kGemmThreads, f.smem, stream>>>(gp);
     int err = check_launch("tc gemm (integer)");
     if (!err && gp.partial)
     {
-        fixup<<<dim3(rest, sums_per_thread), 256, 0, stream>>>(gp);
+        f.fixup<<<dim3((unsigned) (ntasks % sms), f.sums), 256, 0, stream>>>(
+                gp);
         err = check_launch("tc gemm (integer, last wave)");
     }
     if (ev_stop) cudaEventRecord(ev_stop, stream);
     if (to_free) scratch_free(to_free, stream);
     return err;
-}
-
-int launch_gemm_l6(GemmParams& gp, const PartialRoom& room,
-        cudaStream_t stream)
-{
-    return launch_integer(gemm_l6_kernel, gemm_l6_smem_bytes(),
-            fixup_l6_kernel, 8, kL6PartialWords, 1.8, gp, (long long) gp.nrb * (gp.nrb + 1) *
-            gp.num_problems, room, stream);
 }
 
 int launch_gemm(GemmParams& gp, cudaStream_t stream,
@@ -3342,9 +3401,7 @@ int launch_gemm(GemmParams& gp, cudaStream_t stream,
         // square tiles (the integer image's only shape)
         g_last_arith.store(8);
         g_last_tile.store(128);
-        return launch_integer(gemm_i8_kernel, gemm_i8_smem_bytes(),
-                fixup_i8_kernel, 16, kI8PartialWords, 0.72, gp, square, room,
-                stream);
+        return launch_integer(false, gp, room, stream);
     }
     const long long wide_n = (long long) wide_tiles(gp.nrb) *
             gp.num_problems;
@@ -3455,8 +3512,8 @@ int jones_block(int casa, int num_sources, int num_stations, int offset_out,
         const double* jones, const double* I, const double* Q,
         const double* U, const double* V, const double* station_u,
         const double* station_v, double uv_min_lambda, double uv_max_lambda,
-        double inv_wavelength, double* vis, uint8_t* ws, cudaStream_t s,
-        bool pool = true)
+        double inv_wavelength, double* vis, uint8_t* ws,
+        const PartialRoom& room, cudaStream_t s)
 {
     Header* hdr = reinterpret_cast<Header*>(ws);
     // the status words start at zero; the image is rewritten
@@ -3513,8 +3570,6 @@ int jones_block(int casa, int num_sources, int num_stations, int offset_out,
     gp.inv_wavelength = nullptr; gp.kw_scalar = inv_wavelength;
     gp.uv_min = uv_min_lambda; gp.uv_max = uv_max_lambda;
     gp.casa = casa; gp.err = &hdr->err; gp.autos = nullptr;
-    PartialRoom room;
-    room.pool = pool;
     return launch_gemm(gp, s, room);
 }
 
@@ -3531,7 +3586,8 @@ int l6_block(int casa, int num_sources, int num_stations, int offset_out,
         const double* jones, const double* I, const double* Q,
         const double* U, const double* V, const double* station_u,
         const double* station_v, double uv_min_lambda, double uv_max_lambda,
-        double inv_wavelength, double* vis, uint8_t* ws, cudaStream_t s)
+        double inv_wavelength, double* vis, uint8_t* ws,
+        const PartialRoom& room, cudaStream_t s)
 {
     bool wide_fits = false, pair_fits = false;
     int err = device_setup(wide_fits, pair_fits);
@@ -3569,7 +3625,7 @@ int l6_block(int casa, int num_sources, int num_stations, int offset_out,
     gp.inv_wavelength = nullptr; gp.kw_scalar = inv_wavelength;
     gp.uv_min = uv_min_lambda; gp.uv_max = uv_max_lambda;
     gp.casa = casa; gp.err = &hdr->err; gp.autos = nullptr;
-    return launch_gemm_l6(gp, PartialRoom(), s);
+    return launch_integer(true, gp, room, s);
 }
 
 // Workspace of the FP32 entry point: Header, order tables, the integer
@@ -3588,7 +3644,7 @@ int tcf_block(int casa, int num_sources, int num_stations, int offset_out,
         const float* jones, const float* I, const float* Q, const float* U,
         const float* V, const float* station_u, const float* station_v,
         double uv_min_lambda, double uv_max_lambda, double inv_wavelength,
-        float* vis, uint8_t* ws, cudaStream_t s)
+        float* vis, uint8_t* ws, const PartialRoom& room, cudaStream_t s)
 {
     bool wide_fits = false, pair_fits = false;
     int err = device_setup(wide_fits, pair_fits);
@@ -3638,7 +3694,7 @@ int tcf_block(int casa, int num_sources, int num_stations, int offset_out,
     gp.inv_wavelength = nullptr; gp.kw_scalar = inv_wavelength;
     gp.uv_min = uv_min_lambda; gp.uv_max = uv_max_lambda;
     gp.casa = casa; gp.err = &hdr->err; gp.autos = nullptr;
-    if ((err = launch_gemm(gp, s))) return err;
+    if ((err = launch_gemm(gp, s, room))) return err;
     const size_t n = nbl * 8;
     const int grid = (int) std::min<size_t>((n + 255) / 256,
             (size_t) num_sms() * 8);
@@ -3673,14 +3729,16 @@ int correlate_block_l6(int casa, int num_sources, int num_stations,
     {
         group = kept_group(num_problems, kHeaderBytes + tb, img, s);
     }
-    int err = get_workspace(workspace, workspace_bytes,
-            kHeaderBytes + tb + (size_t) group * img, s);
+    const size_t need = kHeaderBytes + tb + (size_t) group * img;
+    int err = get_workspace(workspace, workspace_bytes, need, partial_room(
+            true, num_stations, num_sources, num_problems, group), s);
     if (err) return err;
     bool wide_fits = false, pair_fits = false;
     if ((err = device_setup(wide_fits, pair_fits))) return err;
     uint8_t* ws = reinterpret_cast<uint8_t*>(workspace);
     Header* hdr = reinterpret_cast<Header*>(ws);
     uint8_t* W = ws + kHeaderBytes + tb;
+    const PartialRoom room(workspace, workspace_bytes, need);
     if (cudaMemsetAsync(hdr, 0, sizeof(Header), s) != cudaSuccess)
     {
         set_last_error("tc64 header clear", cudaGetLastError());
@@ -3720,7 +3778,7 @@ int correlate_block_l6(int casa, int num_sources, int num_stations,
         gp.inv_wavelength = inv_wavelength; gp.kw_scalar = 0.0;
         gp.uv_min = uv_min_lambda; gp.uv_max = uv_max_lambda;
         gp.casa = casa; gp.err = &hdr->err; gp.autos = autos;
-        if ((err = launch_gemm_l6(gp, PartialRoom(), s))) return err;
+        if ((err = launch_integer(true, gp, room, s))) return err;
     }
     return 0;
 }
@@ -3755,11 +3813,13 @@ int oskb_cross_correlate_tc_d(int casa, int num_sources, int num_stations,
     const size_t need = oskb_cross_correlate_tc_workspace_bytes(num_sources,
             num_stations);
     cudaStream_t s = as_stream(stream);
-    int err = get_workspace(workspace, workspace_bytes, need, s);
+    int err = get_workspace(workspace, workspace_bytes, need, arith_i8() ?
+            partial_room(false, num_stations, num_sources, 1, 1) : 0, s);
     if (err) return err;
     return jones_block(casa, num_sources, num_stations, offset_out, jones, I,
             Q, U, V, station_u, station_v, uv_min_lambda, uv_max_lambda,
-            inv_wavelength, vis, reinterpret_cast<uint8_t*>(workspace), s);
+            inv_wavelength, vis, reinterpret_cast<uint8_t*>(workspace),
+            PartialRoom(workspace, workspace_bytes, need), s);
 }
 
 size_t oskb_cross_correlate_tc_f_workspace_bytes(int num_sources,
@@ -3785,11 +3845,13 @@ int oskb_cross_correlate_tc_f(int casa, int num_sources, int num_stations,
     const size_t need = oskb_cross_correlate_tc_f_workspace_bytes(
             num_sources, num_stations);
     cudaStream_t s = as_stream(stream);
-    int err = get_workspace(workspace, workspace_bytes, need, s);
+    int err = get_workspace(workspace, workspace_bytes, need, partial_room(
+            false, num_stations, num_sources, 1, 1), s);
     if (err) return err;
     return tcf_block(casa, num_sources, num_stations, offset_out, jones, I, Q,
             U, V, station_u, station_v, uv_min_lambda, uv_max_lambda,
-            inv_wavelength, vis, reinterpret_cast<uint8_t*>(workspace), s);
+            inv_wavelength, vis, reinterpret_cast<uint8_t*>(workspace),
+            PartialRoom(workspace, workspace_bytes, need), s);
 }
 
 size_t oskb_cross_correlate_tc64_workspace_bytes(int num_sources,
@@ -3813,11 +3875,13 @@ int oskb_cross_correlate_tc64_d(int casa, int num_sources, int num_stations,
     const size_t need = oskb_cross_correlate_tc64_workspace_bytes(
             num_sources, num_stations);
     cudaStream_t s = as_stream(stream);
-    int err = get_workspace(workspace, workspace_bytes, need, s);
+    int err = get_workspace(workspace, workspace_bytes, need, partial_room(
+            true, num_stations, num_sources, 1, 1), s);
     if (err) return err;
     return l6_block(casa, num_sources, num_stations, offset_out, jones, I, Q,
             U, V, station_u, station_v, uv_min_lambda, uv_max_lambda,
-            inv_wavelength, vis, reinterpret_cast<uint8_t*>(workspace), s);
+            inv_wavelength, vis, reinterpret_cast<uint8_t*>(workspace),
+            PartialRoom(workspace, workspace_bytes, need), s);
 }
 
 size_t oskb_correlate_block_tc64_workspace_bytes(int num_sources,
@@ -3949,7 +4013,7 @@ int correlate_block(int casa, int num_sources, int num_stations,
         double uv_max_lambda, double* vis, void* workspace,
         size_t workspace_bytes, void* stream,
         void (*after_group)(void* ctx, int p0, int np), void* ctx,
-        double* autos, int form)
+        double* autos, int form, bool pool)
 {
     if (num_sources < 0 || num_stations < 0 || num_times < 0 ||
             num_channels < 0)
@@ -3979,12 +4043,15 @@ int correlate_block(int casa, int num_sources, int num_stations,
                 as_stream(stream));
     }
     cudaStream_t s = as_stream(stream);
-    int err = get_workspace(workspace, workspace_bytes,
-            kHeaderBytes + tb + (size_t) group * img, s);
+    const size_t need = kHeaderBytes + tb + (size_t) group * img;
+    int err = get_workspace(workspace, workspace_bytes, need, i8 ?
+            partial_room(false, num_stations, num_sources, num_problems,
+            group) : 0, s);
     if (err) return err;
     uint8_t* ws = reinterpret_cast<uint8_t*>(workspace);
     Header* hdr = reinterpret_cast<Header*>(ws);
     uint8_t* W = ws + kHeaderBytes + tb;
+    const PartialRoom room(workspace, workspace_bytes, need, pool);
     if (cudaMemsetAsync(hdr, 0, sizeof(Header), s) != cudaSuccess)
     {
         set_last_error("tc header clear", cudaGetLastError());
@@ -4043,10 +4110,6 @@ int correlate_block(int casa, int num_sources, int num_stations,
         gp.inv_wavelength = inv_wavelength; gp.kw_scalar = 0.0;
         gp.uv_min = uv_min_lambda; gp.uv_max = uv_max_lambda;
         gp.casa = casa; gp.err = &hdr->err; gp.autos = autos;
-        PartialRoom room;
-        room.tail = W + (size_t) group * img;
-        room.tail_bytes = workspace_bytes - (kHeaderBytes + tb +
-                (size_t) group * img);
         if ((err = launch_gemm(gp, s, room))) return err;
         if (after_group) after_group(ctx, p0, np);
     }
@@ -4057,12 +4120,19 @@ template int correlate_block<float>(int, int, int, int, int, const float*,
         const double*, const double*, const double*, const double*,
         const double*, const double*, const double*, const double*,
         const double*, double, double, double*, void*, size_t, void*,
-        void (*)(void*, int, int), void*, double*, int);
+        void (*)(void*, int, int), void*, double*, int, bool);
 template int correlate_block<double>(int, int, int, int, int, const double*,
         const double*, const double*, const double*, const double*,
         const double*, const double*, const double*, const double*,
         const double*, double, double, double*, void*, size_t, void*,
-        void (*)(void*, int, int), void*, double*, int);
+        void (*)(void*, int, int), void*, double*, int, bool);
+
+size_t block_room(int num_sources, int num_stations, int num_problems,
+        int group)
+{
+    return partial_room(false, num_stations, num_sources, num_problems,
+            group);
+}
 
 int setup_device()
 {
@@ -4105,6 +4175,11 @@ int oskb_tc_timing_read(double* total_ms, int* launches)
 int oskb_tc_tile_columns(void)
 {
     return g_last_tile.load();
+}
+
+int oskb_tc_last_wave_runs(void)
+{
+    return g_last_pieces.load();
 }
 
 int oskb_tc_arithmetic(void)
@@ -4222,7 +4297,7 @@ extern "C" int oskb_cross_correlate_tc_noalloc_d(int casa, int num_sources,
     return jones_block(casa, num_sources, num_stations, offset_out, jones, I,
             Q, U, V, station_u, station_v, uv_min_lambda, uv_max_lambda,
             inv_wavelength, vis, reinterpret_cast<uint8_t*>(scratch),
-            as_stream(stream), false);
+            PartialRoom(nullptr, 0, 0, false), as_stream(stream));
 }
 
 // Status words of the last allocation-free call on the current device: the

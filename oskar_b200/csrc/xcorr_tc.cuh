@@ -23,7 +23,10 @@ enum Form
 // visibilities (for example their download) while later groups compute;
 // autos (if set) receives the auto-correlations from the same contraction
 // ([time][channel][station][2x2], added). E is FP32 or FP64 (float or
-// double instantiations); form fixes the contraction form.
+// double instantiations); form fixes the contraction form; pool: partial sums
+// of a split last wave may come from the scratch pool where the workspace has
+// no room for them (not for work that is timed for its later replay from a
+// graph, where the pool is not used).
 template <typename TE>
 int correlate_block(int casa, int num_sources, int num_stations,
         int num_times, int num_channels, const TE* E, const double* l,
@@ -33,7 +36,12 @@ int correlate_block(int casa, int num_sources, int num_stations,
         double uv_max_lambda, double* vis, void* workspace,
         size_t workspace_bytes, void* stream,
         void (*after_group)(void* ctx, int p0, int np), void* ctx,
-        double* autos = nullptr, int form = kFormDefault);
+        double* autos = nullptr, int form = kFormDefault, bool pool = true);
+
+// Bytes behind the operand images of a workspace for groups of `group`
+// problems that the integer form's split last wave uses.
+size_t block_room(int num_sources, int num_stations, int num_problems,
+        int group);
 
 // The per-device launch set-up of the contraction kernels (shared-memory
 // opt-ins), done before a stream capture so that none happens inside it.
