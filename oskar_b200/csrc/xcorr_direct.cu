@@ -780,46 +780,62 @@ int tiles_for(int num_st)
     return nb * (nb + 1) / 2;
 }
 
-// Number of source slices for `items` tiles of `chunks` source chunks each on
-// `slots` resident CTAs: the one that minimises the waves of CTAs times the
-// chunks of a slice plus a fixed cost per slice, about two chunks' time
-// (filling the pipeline, and writing and reducing its partial sums of `bytes`
-// bytes). Few long slices that fill the slots once beat many short ones
-// where the tiles take equal time: 128 stations (10 tiles) x 12,000 sources
-// in 14 slices instead of 119. Tiles with dead patches take less (work: the
-// sum in whole tiles), and then more slices than slots even out: the
-// estimate is half a slice beyond the average.
-int choose_slices(long long items, double work, int chunks, int slots,
+// Number of source slices for `items` tiles of `chunks` source chunks each:
+// the one with the least estimated time, in units of a CTA's time per chunk.
+//  - The busiest SM's CTAs one after the other; of a kernel with two
+//    resident per SM (pairs) two take 1.6 times one's time. Tiles with dead patches take less than others (work: the sum in
+//    whole tiles, less than items); the CTAs then even out, and the estimate
+//    is half a slice beyond the average.
+//  - Two chunks' time per slice on that SM: filling the pipeline, storing the
+//    partial sums.
+//  - The sum over the slices, about 0.07 us each: 0.06 of a chunk of the
+//    scalar kernel (1.3 us), 0.02 of the others' (2 to 6 us).
+// Against the best of all counts, at 11 shapes of 16 to 351 stations x 500 to
+// 30,000 sources x both types, with and without smearing, the counts it takes
+// are 1 % slower on average and 15 % at most (197 stations x 800 sources,
+// FP64 smearing, 5 slices for 6). 128 x 12,000 FP64 points (10 tiles): 29
+// slices in two rounds, 332 us; 14 in one are as fast.
+int choose_slices(long long items, double work, bool pairs, int chunks,
         size_t bytes)
 {
-    constexpr int kFixed = 2;
+    constexpr double kFixed = 2.0, kPair = 1.6;
     constexpr size_t kMostBytes = (size_t) 512 << 20;
-    const int most = (int) min((long long) chunks, (8LL * slots + items - 1)
-            / items);
+    const double per_slice = pairs ? 0.06 : 0.02;
+    const int sms = num_sms();
+    const int most = (int) min((long long) chunks, ((pairs ? 16LL : 8LL) *
+            sms + items - 1) / items);
     int best = 1;
     double best_cost = 0;
-    for (int s = 1; s <= most && (s == 1 || s * bytes <= kMostBytes); ++s)
+    for (int len = chunks; len >= 1; )
     {
-        const int len = (chunks + s - 1) / s;
-        if ((chunks + len - 1) / len != s) continue;
-        const long long waves = (items * s + slots - 1) / slots;
-        const double even = work < (double) items ? max(1.0, work * s / slots
-                + 0.5) : (double) waves;
-        const double cost = (waves > 1 ? min(even, (double) waves) : 1.0) *
-                len + (s > 1 ? (double) (waves * kFixed) : 0.0);
+        // the fewest slices of at most len chunks
+        const int s = (chunks + len - 1) / len;
+        if (s > most || (s > 1 && s * bytes > kMostBytes)) break;
+        const long long ctas = (items * s + sms - 1) / sms;
+        double rounds = (double) ctas;
+        if (pairs)
+            rounds = (double) (ctas / 2) * kPair + (double) (ctas % 2);
+        else if (work < (double) items)
+            rounds = min(rounds, max(1.0, work * s / sms + 0.5));
+        const double cost = rounds * len + (s > 1 ? (double) ctas * kFixed +
+                s * per_slice : 0.0);
         if (s == 1 || cost < best_cost)
         {
             best = s;
             best_cost = cost;
         }
+        // the longest chunks of one slice more
+        len = min(len - 1, (chunks + s) / (s + 1));
     }
     return best;
 }
 
 // Work of a smearing launch's tiles, in whole tiles: the share of the 8 x 8
-// patches that hold a baseline.
+// patches that hold a baseline (a single tile counts whole: its slices all
+// take the same time).
 double smear_tiles(int num_st)
 {
+    if (num_st <= kTile) return 1.0;
     const double n = (num_st + 7) / 8;
     return n * (n + 1) / 2 / 16;
 }
@@ -836,17 +852,18 @@ int xcorr_dispatch(bool casa, bool gauss, XcorrParams<T> p,
     if ((uintptr_t) p.jones % Staging<T, MATRIX>::COPY != 0)
         return OSKB_ERR_INVALID_ARGUMENT;
     const int tiles = tiles_for(p.num_st);
-    // CTAs that run at a time: one per SM for the tensor-pipe and smearing
-    // kernels, two for the register-tiled one in FP64
     const bool dmma = use_dmma<T, MATRIX>(gauss, bw, ts);
-    const int per_sm = sizeof(T) == 8 && !dmma && !gauss && !bw && !ts ? 2 :
-            1;
+    // two CTAs per SM: the register-tiled kernel without smearing, scalar or
+    // FP64 (100 to 128 registers); its FP32 matrix form (170) and the
+    // tensor-pipe and smearing kernels have one
+    const bool pairs = !dmma && !gauss && !bw && !ts && (!MATRIX ||
+            sizeof(T) == 8);
     const int chunks = (p.num_src + kChunk - 1) / kChunk;
     const size_t slice_bytes = (size_t) p.num_st * (p.num_st - 1) / 2 *
             (MATRIX ? 8 : 2) * sizeof(double);
     int slices = choose_slices(tiles, gauss || bw || ts ?
-            smear_tiles(p.num_st) : (double) tiles, chunks,
-            per_sm * num_sms(), slice_bytes);
+            smear_tiles(p.num_st) : (double) tiles, pairs, chunks,
+            slice_bytes);
     if (const char* e = getenv("OSKB_XCORR_SLICES")) slices = max(1, atoi(e));
     int slice_len = (p.num_src + slices - 1) / slices;
     slice_len = (slice_len + kChunk - 1) / kChunk * kChunk;
@@ -1025,8 +1042,8 @@ int block_dispatch(bool casa, bool gauss, bool bw, bool ts, XcorrParams<T> p,
     {
         const long long tc = (long long) p.num_times * p.num_channels;
         int slices = choose_slices(tc_items, gauss || bw || ts ?
-                tc * smear_tiles(p.num_st) : (double) tc_items,
-                (p.num_src + kChunk - 1) / kChunk, num_sms(), (size_t) tc *
+                tc * smear_tiles(p.num_st) : (double) tc_items, false,
+                (p.num_src + kChunk - 1) / kChunk, (size_t) tc *
                 p.num_st * (p.num_st - 1) / 2 * 8 * sizeof(double));
         if (slices > 1)
         {

@@ -1,0 +1,82 @@
+"""The number of source slices a direct cross-correlation takes by itself
+(the rule in csrc/xcorr_direct.cu) against other numbers of slices set through
+OSKB_XCORR_SLICES: no more than 1.25 times the time of the best of a few, for
+the kernels it serves (tensor pipe, register tiles with one and with two CTAs
+per SM, smearing) at shapes of one tile, few and many, few and many sources.
+Device times of calls replayed from a graph (repeats agree to about 1 %; the
+rule's own estimate is within 15 % of the best over its ranges)."""
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = [pytest.mark.gpu,
+              pytest.mark.skipif(not torch.cuda.is_available(),
+                                 reason="needs a CUDA device")]
+
+import oskar_b200 as ob  # noqa: E402
+
+ENV = "OSKB_XCORR_SLICES"
+
+
+def microseconds(call, calls=8):
+    s = torch.cuda.Stream()
+    with torch.cuda.stream(s):
+        call()
+        s.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=s):
+            for _ in range(calls):
+                call()
+        times = []
+        for _ in range(6):
+            a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            a.record(s)
+            g.replay()
+            b.record(s)
+            b.synchronize()
+            times.append(a.elapsed_time(b) * 1e3 / calls)
+    del g
+    return min(times[1:])
+
+
+@pytest.mark.parametrize("real", [torch.float64, torch.float32])
+@pytest.mark.parametrize("kind", ["matrix", "scalar", "smear"])
+@pytest.mark.parametrize("nst,nsrc,slices", [
+    (16, 3000, (47, 75, 125)), (30, 1000, (25, 42, 63)),
+    (30, 30000, (75, 145, 290)), (100, 20000, (14, 29, 44)),
+    (197, 4001, (5, 10, 21))])
+def test_rule_against_fixed_counts(real, kind, nst, nsrc, slices,
+                                   monkeypatch):
+    g = torch.Generator(device="cuda")
+    g.manual_seed(nst)
+
+    def rand(*shape):
+        return torch.rand(shape, generator=g, device="cuda", dtype=real)
+
+    matrix = kind == "matrix"
+    l, m = (rand(nsrc) - 0.5) * 0.2, (rand(nsrc) - 0.5) * 0.2
+    n = torch.sqrt(1 - l * l - m * m)
+    flux = [rand(nsrc) + 0.2] + [rand(nsrc) * 0.1 for _ in range(3)]
+    jones = rand(nst, nsrc, 8 if matrix else 2)
+    u, v, w = ((rand(nst) - 0.5) * 2000 for _ in range(3))
+    vis = torch.zeros((nst * (nst - 1) // 2, 8 if matrix else 2),
+                      dtype=real, device="cuda")
+    name = "oskb_cross_correlate_%s%s" % (
+        "" if matrix else "scalar_", "d" if real == torch.float64 else "f")
+    smear = (1e-3, 10.0) if kind == "smear" else (0.0, 0.0)
+
+    def call():
+        ob.call(name, 0, 0, nsrc, nst, 0, jones,
+                *(flux if matrix else flux[:1]), l, m, n, None, None, None,
+                u, v, w, u, v, 0.0, 3e38, 0.37, *smear, 0.3, -0.5, vis,
+                ob.stream_ptr())
+
+    monkeypatch.delenv(ENV, raising=False)
+    own = microseconds(call)
+    best = None
+    for k in slices:
+        monkeypatch.setenv(ENV, str(k))
+        t = microseconds(call)
+        best = t if best is None else min(best, t)
+    monkeypatch.delenv(ENV)
+    own = min(own, microseconds(call))
+    assert own <= 1.25 * best, (own, best)
