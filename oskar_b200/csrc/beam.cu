@@ -294,16 +294,19 @@ struct BeamArgs
 // (planar) against 21 with a complex weight and the 128-entry table.
 template <typename T, bool IS3D, int NT, int ND>
 __device__ __forceinline__ void station_beam_item(BeamSmem<T, IS3D, NT>& sm,
-        const BeamArgs<T>& arg, int st, int d_first)
+        const BeamArgs<T>& arg, int st, unsigned d_first)
 {
     typedef typename vec2<T>::type T2;
     typedef Trig<T> Tr;
-    const int num_elements = arg.num_elements, num_dir = arg.num_dir;
+    const int num_elements = arg.num_elements;
+    // (unsigned: a block may reach past the largest int)
+    const unsigned num_dir = arg.num_dir;
     const BeamFlags& flags = arg.flags;
     const TypeParams<T>& tp = arg.tp;
     const double* beam_enu = arg.beam_enu;
     const int rows = arg.rows;
-    const int d0 = d_first + threadIdx.x, threads = blockDim.x;
+    const unsigned d0 = d_first + threadIdx.x;
+    const int threads = blockDim.x;
     const size_t el0 = (size_t) st * num_elements;
     const size_t dir0 = arg.directions_per_station ? (size_t) st * num_dir : 0;
     const int per_dir = flags.scalar ? 1 : 4;
@@ -316,7 +319,7 @@ __device__ __forceinline__ void station_beam_item(BeamSmem<T, IS3D, NT>& sm,
 #pragma unroll
         for (int j = 0; j < ND; ++j)
         {
-            const int d = d0 + j * threads;
+            const unsigned d = d0 + j * threads;
             if (d < num_dir)
                 for (int k = 0; k < per_dir; ++k)
                     out[(size_t) per_dir * d + k] = T2{(T) 0, (T) 0};
@@ -337,7 +340,7 @@ __device__ __forceinline__ void station_beam_item(BeamSmem<T, IS3D, NT>& sm,
 #pragma unroll
     for (int j = 0; j < ND; ++j)
     {
-        const int d = d0 + j * threads;
+        const unsigned d = d0 + j * threads;
         X[j] = Y[j] = Z[j] = 0;
         if (d < num_dir)
         {
@@ -502,7 +505,7 @@ __device__ __forceinline__ void station_beam_item(BeamSmem<T, IS3D, NT>& sm,
     const T array_scale = flags.normalise_array ?
             (T) (1.0 / num_elements) : (T) 1;
 
-    // Final normalisation: amplitude of the arg.beam in the normalisation
+    // Final normalisation: amplitude of the beam in the normalisation
     // direction (block reduction of its array factors first).
     T final_scale = (T) 1;
     if (flags.normalise_final)
@@ -606,7 +609,7 @@ __device__ __forceinline__ void station_beam_item(BeamSmem<T, IS3D, NT>& sm,
 #pragma unroll 1
     for (int j = 0; j < ND; ++j)
     {
-        const int d = d0 + j * threads;
+        const unsigned d = d0 + j * threads;
         if (d >= num_dir) break;
         T2* o = out + (size_t) per_dir * d;
         T x = X[0], y = Y[0], z = Z[0], fr[NT], fi[NT];
@@ -685,35 +688,30 @@ __device__ __forceinline__ void station_beam_item(BeamSmem<T, IS3D, NT>& sm,
 
 // One CTA takes items in turn, with its table filled once: first `full`
 // (station, block of threads x BIG directions) items in whole rounds of the
-// grid, then the rest in quarters or halves of threads x SMALL directions,
-// so that the last round is short: at 128 stations x 12,000 directions a
-// grid of 296 has 5.2 rounds of 1,024 directions, and a whole sixth round
-// would idle most of the chip. More directions per thread share the staged
-// element terms (FP64: 629 us with four against 668 us with one on that
-// shape, before the split).
+// grid, then the rest of the directions in parts of threads x SMALL, so that
+// the last round is short: at 128 stations x 12,000 directions a grid of 296
+// has 5.2 rounds of 1,024 directions, and a whole sixth round would idle most
+// of the chip. More directions per thread share the staged element terms
+// (FP64: 629 us with four against 668 us with one on that shape, before the
+// split). Parts [first, total) are numbered station by station, `parts` each,
+// so none is empty (numbered block by block, half of the CTAs met the empty
+// parts of stations just beyond a block: 393 stations x 513 elements x 1,025
+// directions FP64 664 us).
 template <typename T, bool IS3D, int NT, int BIG, int SMALL>
 __global__ void __launch_bounds__(kThreads, kCtasPerSm)
-station_beam_kernel(const __grid_constant__ BeamArgs<T> arg, int blocks,
-        int items, int full)
+station_beam_kernel(const __grid_constant__ BeamArgs<T> arg, unsigned blocks,
+        unsigned full, unsigned parts, unsigned first, unsigned total)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     BeamSmem<T, IS3D, NT>& sm =
             *reinterpret_cast<BeamSmem<T, IS3D, NT>*>(smem_raw);
     Trig<T>::fill(sm.table);
-    for (int item = blockIdx.x; item < full; item += gridDim.x)
+    for (unsigned item = blockIdx.x; item < full; item += gridDim.x)
         station_beam_item<T, IS3D, NT, BIG>(sm, arg, item / blocks,
-                item % blocks * ((int) blockDim.x * BIG));
-    // the rest part by part, so that the empty ones past the last direction
-    // come last
-    const int rest = items - full;
-    for (int n = blockIdx.x; n < rest * (BIG / SMALL); n += gridDim.x)
-    {
-        const int item = full + n % rest, part = n / rest;
-        const int d = item % blocks * ((int) blockDim.x * BIG) + part *
-                ((int) blockDim.x * SMALL);
-        if (d < arg.num_dir)
-            station_beam_item<T, IS3D, NT, SMALL>(sm, arg, item / blocks, d);
-    }
+                item % blocks * (blockDim.x * BIG));
+    for (unsigned n = first + blockIdx.x; n < total; n += gridDim.x)
+        station_beam_item<T, IS3D, NT, SMALL>(sm, arg, n / parts,
+                n % parts * (blockDim.x * SMALL));
 }
 
 // Final normalisation of a station beam evaluated one feed per launch:
@@ -890,18 +888,20 @@ int station_beam_aa(int num_stations, int num_elements, const T* el_x,
     const int per_sm = std::min(sizeof(T) == 8 ? kCtasPerSm : 2 * kCtasPerSm,
             kCtasPerSm * kThreads / threads);
     const int big = dirs_big<T>(num_element_types);
-    const int parts = big / kDirsSmall<T>;
     const int blocks = (int) (((long long) num_directions + threads * big -
             1) / (threads * big));
+    const int parts = (int) (((long long) num_directions + threads * small -
+            1) / (threads * small));
     const long long items = (long long) blocks * num_stations;
-    if (items > INT_MAX / parts) return OSKB_ERR_INVALID_ARGUMENT;
+    const long long total = (long long) parts * num_stations;
+    if (total > INT_MAX) return OSKB_ERR_INVALID_ARGUMENT;
     const int slots = per_sm * sms;
     // whole rounds of big items, unless their blocks would be a quarter
     // empty or more
     const bool dense = 4LL * num_directions >= 3LL * blocks * threads * big;
     const int full = dense ? (int) (items / slots * slots) : 0;
-    const int grid = full ? slots : (int) std::min<long long>(slots, items *
-            parts);
+    const int first = full / blocks * parts + full % blocks * (big / small);
+    const int grid = full ? slots : (int) std::min<long long>(slots, total);
     const BeamArgs<T> arg = {num_elements, el_x, el_y, el_z, meas_x, meas_y,
             meas_z, cable, weight_factors, element_type, orientation_x,
             orientation_y, tp, flags, wavenumber, beam_enu, norm_enu,
@@ -915,7 +915,8 @@ int station_beam_aa(int num_stations, int num_elements, const T* el_x,
         const int smem = (int) sizeof(BeamSmem<T, D, NT>);                   \
         cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, \
                 smem);                                                       \
-        k<<<grid, threads, smem, s>>>(arg, blocks, (int) items, full);       \
+        k<<<grid, threads, smem, s>>>(arg, blocks, full, parts, first,       \
+                (unsigned) total);                                           \
     }
 #define OSKB_BEAM_NT(D)                                                      \
     switch (num_element_types)                                               \
