@@ -9,18 +9,17 @@
 // (define_dftw_m2m.h:24-107), horizon blanking
 // (define_blank_below_horizon.h:15-29) and final normalisation
 // (define_mem_normalise.h:31-51). The reference runs these as six kernels
-// with five round trips through a per-station signal buffer; here one thread
-// owns one (station, direction) and the pieces stay in registers.
+// with five round trips through a per-station signal buffer; here a thread
+// owns one to four directions of a station and the pieces stay in registers.
 //
 // With a single element type the weighted DFT of the element signals is
 // pattern(dir) x AF(dir), AF = sum_e w_e exp(i k r_e . dir): the pattern is
 // evaluated once per direction and the element loop carries only the array
-// factor (one sincos and one complex multiply-add per element-direction).
-// Element weights and positions are staged in shared memory in chunks.
+// factor: per element-direction one phase, which includes the weight's, one
+// table lookup (trig_table.cuh, both precisions) and one real-by-complex
+// multiply-add. Element terms are staged in shared memory in chunks.
 // The normalisation direction's beam (one per station) is recomputed by each
-// CTA cooperatively before the main loop, so there is no second launch.
-// In FP64 the element loops take their phase factors from a shared-memory
-// table (trig_table.cuh) instead of a library sincos per element-direction.
+// CTA cooperatively beside the staging, so there is no second launch.
 #include <algorithm>
 #include <climits>
 
@@ -34,7 +33,7 @@ constexpr int kThreads = 256;
 constexpr int kChunk = 512;
 constexpr int kCtasPerSm = 2;
 // directions per thread: most items, and those of the last round (FP32 works
-// on pairs)
+// on pairs, but on one where a call's directions do not fill the chip)
 template <typename T>
 constexpr int dirs_big(int num_types)
 {
@@ -196,8 +195,17 @@ __device__ __forceinline__ void element_factors(
     const ulonglong2 pg = *reinterpret_cast<const ulonglong2*>(&el.pg[i]);
     float g2;
     unpack2(pg.y, gain, g2);
+    if constexpr (ND == 1)
+    {
+        const float4 p = el.xy[i];
+        float u = fmaf(kY[0], p.z, el.pg[i].x);
+        if (IS3D) u = fmaf(kZ[0], el.z[i].x, u);
+        u = fmaf(kX[0], p.x, u);
+        Trig<float>::sincos(table, u, &sn[0], &cs[0]);
+        return;
+    }
 #pragma unroll
-    for (int j = 0; j < ND; j += 2)
+    for (int j = 0; j + 1 < ND; j += 2)
     {
         f32x2 u = fma2(pack2(kY[j], kY[j + 1]), xy.y, pg.x);
         if (IS3D)
@@ -256,7 +264,10 @@ struct BeamSmem
     ElementTerms<T, IS3D> el;
     int type[NT > 1 ? kChunk : 1];
     T red[2][NT][kThreads / 32];
-    T rot[NT][4];        // element_pattern_rotated's, of the item's station
+    // Of the item's station, per element type: the elements' azimuths, their
+    // cosines and sines (element_pattern_rotated's), the pole normalisation
+    // and the pattern and taper in the normalisation direction.
+    T dphi[NT][2], rot[NT][4], pole[NT], norm_p[NT][4], norm_taper[NT];
     unsigned bound[3];   // largest |x|, |y|, |z| of the chunk, float bits
 };
 
@@ -286,7 +297,35 @@ struct BeamArgs
     T* beam;
 };
 
-// Beam of station st in directions d_first + thread + j kThreads, j < ND.
+// Half f of the terms of element type t of station st (BeamSmem), each by one
+// thread, so that the patterns of all types at the pole and in the
+// normalisation direction take the time of one.
+template <typename T, bool IS3D, int NT>
+__device__ __forceinline__ void station_terms(BeamSmem<T, IS3D, NT>& sm,
+        const BeamArgs<T>& arg, int st, int t, int f, T nX, T nY, T nZ)
+{
+    const T dphi1 = (T) (kPi / 2 - (arg.orientation_x[st * NT + t] + kPi / 2));
+    const T dphi2 = (T) (kPi / 2 - arg.orientation_y[st * NT + t]);
+    sm.dphi[t][f] = f ? dphi2 : dphi1;
+    if constexpr (sizeof(T) == 8)
+        sincos(f ? dphi2 : dphi1, &sm.rot[t][2 * f + 1], &sm.rot[t][2 * f]);
+    // f = 0: the pole; 1: the normalisation direction
+    T p[4] = {};
+    if (f ? arg.flags.normalise_final : arg.flags.normalise_element)
+        type_pattern<T>(arg.tp, t, f ? nX : (T) 0, f ? nY : (T) 0, f ? nZ :
+                (T) 1, f == 0, dphi1, dphi2, arg.flags.swap_xy, p);
+    if (f)
+    {
+        for (int k = 0; k < 4; ++k) sm.norm_p[t][k] = p[k];
+        sm.norm_taper[t] = type_taper<T>(arg.tp, t, nX, nY, nZ);
+    }
+    else
+        // element normalisation: 1 / |pattern at the pole|
+        sm.pole[t] = arg.flags.normalise_element ? (T) 1 /
+                sqrt(half_frobenius<T>(p, 1, 0)) : (T) 1;
+}
+
+// Beam of station st in directions d_first + thread + j threads, j < ND.
 // The weight of an element, f e^{-i k (r_m . b + cable)}, is folded into the
 // element loop as a gain |f| and a phase in table steps, so an
 // element-direction is one phase (2 or 3 multiply-adds), one table phase
@@ -326,32 +365,18 @@ __device__ __forceinline__ void station_beam_item(BeamSmem<T, IS3D, NT>& sm,
         }
         return;
     }
-    // element orientations per (station, type)
-    T dphi1[NT], dphi2[NT];
-#pragma unroll
-    for (int t = 0; t < NT; ++t)
-    {
-        dphi1[t] = (T) (kPi / 2 - (arg.orientation_x[st * NT + t] + kPi / 2));
-        dphi2[t] = (T) (kPi / 2 - arg.orientation_y[st * NT + t]);
-    }
-
-    T X[ND], Y[ND], Z[ND], kX[ND], kY[ND], kZ[ND];
+    T kX[ND], kY[ND], kZ[ND];
     const double k_steps = arg.wavenumber * Tr::kStepsPerRadian;
 #pragma unroll
     for (int j = 0; j < ND; ++j)
     {
         const unsigned d = d0 + j * threads;
-        X[j] = Y[j] = Z[j] = 0;
-        if (d < num_dir)
-        {
-            X[j] = arg.dir_x[dir0 + d];
-            Y[j] = arg.dir_y[dir0 + d];
-            Z[j] = arg.dir_z[dir0 + d];
-        }
+        const bool in = d < num_dir;
         // phase per metre in table steps, rounded once
-        kX[j] = (T) (k_steps * (double) X[j]);
-        kY[j] = (T) (k_steps * (double) Y[j]);
-        kZ[j] = (T) (k_steps * (double) Z[j]);
+        kX[j] = (T) (in ? k_steps * (double) arg.dir_x[dir0 + d] : 0.0);
+        kY[j] = (T) (in ? k_steps * (double) arg.dir_y[dir0 + d] : 0.0);
+        kZ[j] = (T) (IS3D && in ? k_steps * (double) arg.dir_z[dir0 + d] :
+                0.0);
     }
     T nX = 0, nY = 0, nZ = 1;
     if (flags.normalise_final)
@@ -374,23 +399,21 @@ __device__ __forceinline__ void station_beam_item(BeamSmem<T, IS3D, NT>& sm,
 #pragma unroll
         for (int j = 0; j < ND; ++j) ar[j][t] = ai[j][t] = (T) 0;
     }
+    // The station's terms, by lanes of the last warp, which has the fewest
+    // elements to stage: beside the other warps' staging where the element
+    // loop is short, else beside their loops (128 stations x 12,000
+    // directions FP64: 564 us against 576 before the staging).
+    const int lane = threadIdx.x & 31;
+    const int term = threadIdx.x >= threads - 32 && lane < 2 * NT ? lane : -1;
     for (int e0 = 0; e0 < num_elements; e0 += kChunk)
     {
         const int ne = min(kChunk, num_elements - e0);
         __syncthreads();  // table filled; the previous chunk is consumed
         if (threadIdx.x < 3) sm.bound[threadIdx.x] = 0;
-        if (e0 == 0 && threadIdx.x >= 32 && threadIdx.x < 32 + 2 * NT)
-        {
-            const int t = (threadIdx.x - 32) >> 1, f = threadIdx.x & 1;
-            T d1 = 0, s1, c1;
-#pragma unroll
-            for (int k = 0; k < NT; ++k)
-                if (k == t) d1 = f ? dphi2[k] : dphi1[k];
-            sincos(d1, &s1, &c1);
-            sm.rot[t][2 * f] = c1;
-            sm.rot[t][2 * f + 1] = s1;
-        }
         __syncthreads();
+        if (ND == 1 && e0 == 0 && term >= 0)
+            station_terms<T, IS3D, NT>(sm, arg, st, term >> 1, term & 1, nX,
+                    nY, nZ);
         unsigned ex = 0, ey = 0, ez = 0;
         for (int t = threadIdx.x; t < ne; t += threads)
         {
@@ -442,6 +465,9 @@ __device__ __forceinline__ void station_beam_item(BeamSmem<T, IS3D, NT>& sm,
             if (IS3D) atomicMax(&sm.bound[2], ez);
         }
         __syncthreads();
+        if (ND > 1 && e0 == 0 && term >= 0)
+            station_terms<T, IS3D, NT>(sm, arg, st, term >> 1, term & 1, nX,
+                    nY, nZ);
         if (d0 < num_dir)
         {
             // The table covers every phase of the chunk when the largest
@@ -488,20 +514,8 @@ __device__ __forceinline__ void station_beam_item(BeamSmem<T, IS3D, NT>& sm,
         }
     }
 
-    // Element normalisation: 1 / |pattern at the pole|, per type.
-    T pole_scale[NT];
-#pragma unroll
-    for (int t = 0; t < NT; ++t)
-    {
-        pole_scale[t] = (T) 1;
-        if (flags.normalise_element)
-        {
-            T pp[4];
-            type_pattern<T>(tp, t, 0, 0, 1, true, dphi1[t], dphi2[t],
-                    flags.swap_xy, pp);
-            pole_scale[t] = (T) 1 / sqrt(half_frobenius<T>(pp, 1, 0));
-        }
-    }
+    if (ND > 1 && !flags.normalise_final)
+        __syncthreads();   // (else the reduction's) the terms are there
     const T array_scale = flags.normalise_array ?
             (T) (1.0 / num_elements) : (T) 1;
 
@@ -557,12 +571,8 @@ __device__ __forceinline__ void station_beam_item(BeamSmem<T, IS3D, NT>& sm,
 #pragma unroll
             for (int t = 0; t < NT; ++t)
             {
-                T pn[4];
-                type_pattern<T>(tp, t, nX, nY, nZ, false, dphi1[t],
-                        dphi2[t], flags.swap_xy, pn);
-                const T a = sqrt(half_frobenius<T>(pn, 1, 0)) *
-                        type_taper<T>(tp, t, nX, nY, nZ) * pole_scale[t] *
-                        array_scale;
+                const T a = sqrt(half_frobenius<T>(sm.norm_p[t], 1, 0)) *
+                        sm.norm_taper[t] * sm.pole[t] * array_scale;
                 vr += a * nr[t];
                 vi += a * ni[t];
             }
@@ -571,25 +581,15 @@ __device__ __forceinline__ void station_beam_item(BeamSmem<T, IS3D, NT>& sm,
         else if constexpr (NT == 1)
         {
             T pn[4];
-            type_pattern<T>(tp, 0, nX, nY, nZ, false, dphi1[0], dphi2[0],
-                    flags.swap_xy, pn);
-            const T taper = type_taper<T>(tp, 0, nX, nY, nZ);
+#pragma unroll
             for (int k = 0; k < 4; ++k)
-                pn[k] *= pole_scale[0] * taper * array_scale;
+                pn[k] = sm.norm_p[0][k] * (sm.pole[0] * sm.norm_taper[0] *
+                        array_scale);
             final_scale = (T) 1 / sqrt(half_frobenius<T>(pn, nr[0], ni[0]));
         }
         else
         {
             // |sum_t pattern_t AF_t|_F^2 / 2 over the four polarisations
-            T pn[NT][4];
-#pragma unroll
-            for (int t = 0; t < NT; ++t)
-            {
-                type_pattern<T>(tp, t, nX, nY, nZ, false, dphi1[t],
-                        dphi2[t], flags.swap_xy, pn[t]);
-                const T taper = type_taper<T>(tp, t, nX, nY, nZ);
-                for (int k = 0; k < 4; ++k) pn[t][k] *= taper;
-            }
             T amp = 0;
             for (int k = 0; k < 4; ++k)
             {
@@ -597,7 +597,8 @@ __device__ __forceinline__ void station_beam_item(BeamSmem<T, IS3D, NT>& sm,
 #pragma unroll
                 for (int t = 0; t < NT; ++t)
                 {
-                    const T pk = pn[t][k] * pole_scale[t] * array_scale;
+                    const T pk = sm.norm_p[t][k] * sm.norm_taper[t] *
+                            sm.pole[t] * array_scale;
                     vr += pk * nr[t];
                     vi += pk * ni[t];
                 }
@@ -612,7 +613,10 @@ __device__ __forceinline__ void station_beam_item(BeamSmem<T, IS3D, NT>& sm,
         const unsigned d = d0 + j * threads;
         if (d >= num_dir) break;
         T2* o = out + (size_t) per_dir * d;
-        T x = X[0], y = Y[0], z = Z[0], fr[NT], fi[NT];
+        // (read again: kept, they would spill from the element loop)
+        const T x = arg.dir_x[dir0 + d], y = arg.dir_y[dir0 + d],
+                z = arg.dir_z[dir0 + d];
+        T fr[NT], fi[NT];
 #pragma unroll
         for (int t = 0; t < NT; ++t)
         {
@@ -622,66 +626,62 @@ __device__ __forceinline__ void station_beam_item(BeamSmem<T, IS3D, NT>& sm,
 #pragma unroll
         for (int k = 1; k < ND; ++k)
             if (j == k)
-            {
-                x = X[k];
-                y = Y[k];
-                z = Z[k];
 #pragma unroll
                 for (int t = 0; t < NT; ++t)
                 {
                     fr[t] = ar[k][t];
                     fi[t] = ai[k][t];
                 }
-            }
         const bool blank = z < (T) 0;
-        if (flags.scalar)
-        {
-            // pattern amplitude sqrt(sum p_k^2 / 2)
-            // (define_evaluate_dipole_pattern.h:51-75) times the array
-            // factor
-            T2 v{(T) 0, (T) 0};
-#pragma unroll
-            for (int t = 0; t < NT; ++t)
-            {
-                T pt[4];
-                direction_pattern<T>(tp, t, x, y, z, dphi1[t], dphi2[t],
-                        sm.rot[t], flags.swap_xy, pt);
-                const T a = sqrt(half_frobenius<T>(pt, 1, 0)) *
-                        type_taper<T>(tp, t, x, y, z) * pole_scale[t];
-                v.x += a * fr[t] * array_scale;
-                v.y += a * fi[t] * array_scale;
-            }
-            if (blank) v = T2{(T) 0, (T) 0};
-            o[0] = T2{v.x * final_scale, v.y * final_scale};
-            continue;
-        }
-        T p[NT][4];
-#pragma unroll
+        // The reference's order: pattern (normalised), times the weighted
+        // element sum, times the DFT norm, then the final scale. One copy of
+        // the pattern's code for all types: a call of few directions waits
+        // for its instructions, about 3,000 cycles per copy (FP32, 4
+        // stations x 18 elements x 3,614 directions, four types, with the
+        // same for the patterns of station_terms: 26.7 -> 10.8 us).
+        T2 v[4] = {};
+#pragma unroll 1
         for (int t = 0; t < NT; ++t)
         {
-            direction_pattern<T>(tp, t, x, y, z, dphi1[t], dphi2[t],
-                    sm.rot[t], flags.swap_xy, p[t]);
+            T wr = fr[0], wi = fi[0];
+#pragma unroll
+            for (int k = 1; k < NT; ++k)
+                if (t == k)
+                {
+                    wr = fr[k];
+                    wi = fi[k];
+                }
+            T pt[4];
+            direction_pattern<T>(tp, t, x, y, z, sm.dphi[t][0],
+                    sm.dphi[t][1], sm.rot[t], flags.swap_xy, pt);
             const T taper = type_taper<T>(tp, t, x, y, z);
-            for (int k = 0; k < 4; ++k) p[t][k] *= taper;
+            if (flags.scalar)
+            {
+                // pattern amplitude sqrt(sum p_k^2 / 2)
+                // (define_evaluate_dipole_pattern.h:51-75) times the array
+                // factor
+                const T a = sqrt(half_frobenius<T>(pt, 1, 0)) * taper *
+                        sm.pole[t];
+                v[0].x += a * wr * array_scale;
+                v[0].y += a * wi * array_scale;
+                continue;
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+            {
+                const T pk = pt[k] * taper * sm.pole[t];
+                v[k].x += pk * wr * array_scale;
+                v[k].y += pk * wi * array_scale;
+            }
         }
 #pragma unroll
         for (int k = 0; k < 4; ++k)
         {
-            // The reference's order: pattern (normalised), times the
-            // weighted element sum, times the DFT norm, then the final
-            // scale.
-            T2 v{(T) 0, (T) 0};
-#pragma unroll
-            for (int t = 0; t < NT; ++t)
-            {
-                const T pk = p[t][k] * pole_scale[t];
-                v.x += pk * fr[t] * array_scale;
-                v.y += pk * fi[t] * array_scale;
-            }
-            if (blank) v = T2{(T) 0, (T) 0};
-            v.x *= final_scale;
-            v.y *= final_scale;
-            if (rows == 0 || (rows == 1) == (k < 2)) o[k] = v;
+            if (blank) v[k] = T2{(T) 0, (T) 0};
+            v[k].x *= final_scale;
+            v[k].y *= final_scale;
+            if (flags.scalar ? k == 0 : rows == 0 || (rows == 1) == (k < 2))
+                o[k] = v[k];
         }
     }
 }
@@ -693,14 +693,18 @@ __device__ __forceinline__ void station_beam_item(BeamSmem<T, IS3D, NT>& sm,
 // has 5.2 rounds of 1,024 directions, and a whole sixth round would idle most
 // of the chip. More directions per thread share the staged element terms
 // (FP64: 629 us with four against 668 us with one on that shape, before the
-// split). Parts [first, total) are numbered station by station, `parts` each,
-// so none is empty (numbered block by block, half of the CTAs met the empty
-// parts of stations just beyond a block: 393 stations x 513 elements x 1,025
-// directions FP64 664 us).
+// split). The parts are those of the stations from first_station on (the
+// first one's from first_part), the first part of every station before the
+// second and so on: none is empty, and the last ones, which are short, come
+// last and spread over the CTAs. (Numbered so that a station's short or empty
+// parts fell to every second CTA, 393 stations x 513 elements x 1,025
+// directions FP64 took 664 us, now 391.)
 template <typename T, bool IS3D, int NT, int BIG, int SMALL>
-__global__ void __launch_bounds__(kThreads, kCtasPerSm)
+__global__ void __launch_bounds__(kThreads, BIG == 1 && sizeof(T) == 4 ? 1 :
+        kCtasPerSm)
 station_beam_kernel(const __grid_constant__ BeamArgs<T> arg, unsigned blocks,
-        unsigned full, unsigned parts, unsigned first, unsigned total)
+        unsigned full, unsigned first_station, unsigned first_part,
+        unsigned stations, unsigned total)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     BeamSmem<T, IS3D, NT>& sm =
@@ -709,9 +713,13 @@ station_beam_kernel(const __grid_constant__ BeamArgs<T> arg, unsigned blocks,
     for (unsigned item = blockIdx.x; item < full; item += gridDim.x)
         station_beam_item<T, IS3D, NT, BIG>(sm, arg, item / blocks,
                 item % blocks * (blockDim.x * BIG));
-    for (unsigned n = first + blockIdx.x; n < total; n += gridDim.x)
-        station_beam_item<T, IS3D, NT, SMALL>(sm, arg, n / parts,
-                n % parts * (blockDim.x * SMALL));
+    for (unsigned n = blockIdx.x; n < total; n += gridDim.x)
+    {
+        const unsigned st = first_station + n % stations, p = n / stations;
+        if (n % stations != 0 || p >= first_part)
+            station_beam_item<T, IS3D, NT, SMALL>(sm, arg, st,
+                    p * (blockDim.x * SMALL));
+    }
 }
 
 // Final normalisation of a station beam evaluated one feed per launch:
@@ -843,6 +851,111 @@ int make_type_params(int num_types, const double* dipole_length_m,
     return 0;
 }
 
+// Work items of a launch (station_beam_kernel) on `threads` threads per CTA:
+// `full` items of big directions per thread in whole rounds, the rest in
+// parts of small (few: of one, by the kernel that has no other).
+struct BeamSplit
+{
+    int threads, small, few, grid;
+    int blocks, full, first_station, first_part, stations;
+    long long total;   // parts
+};
+
+// CTAs that an SM holds: two tables of 64 KB or four of 32 fit.
+template <typename T>
+int beam_ctas_per_sm(int threads)
+{
+    return std::min(sizeof(T) == 8 ? kCtasPerSm : 2 * kCtasPerSm,
+            kCtasPerSm * kThreads / threads);
+}
+
+// The items of a call. Where its directions do not fill whole rounds of big
+// items, the threads per CTA and the directions per thread of the parts are
+// those of the least estimated time, in units of one element's work on an
+// SM's 256 directions: the rounds of the busiest SM's CTAs (latency of the
+// element loop, of the patterns and of staging the elements), the work of
+// its directions and the table's filling. Constants fitted to the times of
+// 694 shapes of 1 to 512 stations x 16 to 1,024 elements x 200 to 30,000
+// directions x 1 to 4 element types, both precisions, with every choice
+// timed: the choice is 0.5 % above the best on average. Against one direction
+// per thread on 128 threads and the 128-entry table (FP64) or sincosf (FP32)
+// calls of all sizes take 0.77 (FP64) and 0.63 (FP32) of the time; of 900
+// shapes 13 take 1 to 9 % more, and 18 stations x 17 elements x 9,053
+// directions FP32, whose time is the patterns', 24 %.
+template <typename T>
+BeamSplit beam_split(int num_stations, int num_elements, int num_directions,
+        int num_types)
+{
+    constexpr bool f64 = sizeof(T) == 8;
+    const int sms = device_sm_count(), big = dirs_big<T>(num_types);
+    const auto ceil_div = [](long long a, long long b)
+    {
+        return (a + b - 1) / b;
+    };
+    BeamSplit s = {kThreads, kDirsSmall<T>, 0};
+    // whole rounds of big items, unless their blocks would be a quarter
+    // empty or more
+    const int slots = kCtasPerSm * sms;
+    s.blocks = (int) ceil_div(num_directions, kThreads * big);
+    const long long items = (long long) s.blocks * num_stations;
+    if (4LL * num_directions >= 3LL * s.blocks * kThreads * big)
+        s.full = (int) std::min<long long>(items / slots * slots, INT_MAX);
+    if (s.full == 0)
+    {
+        double best = 0;
+        for (int small = kDirsSmall<T>; small >= 1; small /= 2)
+            for (int threads = kThreads; threads >= 64; threads /= 2)
+            {
+                const double ctas = (double) ceil_div(ceil_div(num_directions,
+                        threads * small) * num_stations, sms);
+                const double rounds = ceil(ctas / beam_ctas_per_sm<T>(
+                        threads));
+                const double staging = (double) ceil_div(std::min(
+                        num_elements, kChunk), threads) * std::max(1.0,
+                        (double) num_elements / kChunk);
+                // (FP32: one direction at a time takes 1.3 times its share
+                // of a pair; FP64: warps without directions take less)
+                const double work = f64 ? 1.0 : small == 1 ? 1.3 : small;
+                const double all = ctas * threads, live = std::max<double>(
+                        threads, 32.0 * ceil_div(num_directions, 32 * small) *
+                        num_stations / sms);
+                const double cost = rounds * (small * ((f64 ? 0.08 : 0.4) *
+                        num_elements + (f64 ? 2.4 : 12.0) * num_types) +
+                        40.0 * staging) + (f64 ? 0.68 * all + 0.32 * live :
+                        all) * work / 256.0 * num_elements + (f64 ? 7.5 :
+                        10.0) * 256 / threads;
+                if (best == 0 || cost < best)
+                {
+                    best = cost;
+                    s.threads = threads;
+                    s.small = small;
+                    s.few = small == 1;
+                }
+            }
+    }
+    s.first_station = s.full / s.blocks;
+    s.first_part = s.full % s.blocks * (big / s.small);
+    s.stations = num_stations - s.first_station;
+    s.total = ceil_div(num_directions, s.threads * s.small) * s.stations;
+    s.grid = s.full ? slots : (int) std::min<long long>(s.total,
+            beam_ctas_per_sm<T>(s.threads) * sms);
+    return s;
+}
+
+template <typename T, bool IS3D, int NT>
+void launch_beam(const BeamArgs<T>& arg, const BeamSplit& s,
+        cudaStream_t stream)
+{
+    auto k = station_beam_kernel<T, IS3D, NT, dirs_big<T>(NT), kDirsSmall<T>>;
+    if (s.few)
+        k = station_beam_kernel<T, IS3D, NT, 1, 1>;
+    const int smem = (int) sizeof(BeamSmem<T, IS3D, NT>);
+    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+            smem);
+    k<<<s.grid, s.threads, smem, stream>>>(arg, s.blocks, s.full,
+            s.first_station, s.first_part, s.stations, (unsigned) s.total);
+}
+
 template <typename T>
 int station_beam_aa(int num_stations, int num_elements, const T* el_x,
         const T* el_y, const T* el_z, const T* meas_x, const T* meas_y,
@@ -874,34 +987,9 @@ int station_beam_aa(int num_stations, int num_elements, const T* el_x,
     const double wavenumber = 2.0 * kPi * frequency_hz / c0;
     BeamFlags flags{normalise_element, normalise_array, normalise_final,
             swap_xy, scalar};
-    // Threads per CTA: fewer where blocks of 256 x kDirsSmall directions do
-    // not give every SM one (1 station x 20,000 directions: 79 of them) or
-    // would be half empty; an SM then takes more CTAs (two tables of 64 KB or
-    // four of 32 fit).
-    const int sms = device_sm_count();
-    constexpr int small = kDirsSmall<T>;
-    int threads = kThreads;
-    while (threads > 64 && (num_directions <= threads / 2 * small ||
-            ((long long) num_directions + threads * small - 1) /
-            (threads * small) * num_stations < sms))
-        threads /= 2;
-    const int per_sm = std::min(sizeof(T) == 8 ? kCtasPerSm : 2 * kCtasPerSm,
-            kCtasPerSm * kThreads / threads);
-    const int big = dirs_big<T>(num_element_types);
-    const int blocks = (int) (((long long) num_directions + threads * big -
-            1) / (threads * big));
-    const int parts = (int) (((long long) num_directions + threads * small -
-            1) / (threads * small));
-    const long long items = (long long) blocks * num_stations;
-    const long long total = (long long) parts * num_stations;
-    if (total > INT_MAX) return OSKB_ERR_INVALID_ARGUMENT;
-    const int slots = per_sm * sms;
-    // whole rounds of big items, unless their blocks would be a quarter
-    // empty or more
-    const bool dense = 4LL * num_directions >= 3LL * blocks * threads * big;
-    const int full = dense ? (int) (items / slots * slots) : 0;
-    const int first = full / blocks * parts + full % blocks * (big / small);
-    const int grid = full ? slots : (int) std::min<long long>(slots, total);
+    const BeamSplit split = beam_split<T>(num_stations, num_elements,
+            num_directions, num_element_types);
+    if (split.total > INT_MAX) return OSKB_ERR_INVALID_ARGUMENT;
     const BeamArgs<T> arg = {num_elements, el_x, el_y, el_z, meas_x, meas_y,
             meas_z, cable, weight_factors, element_type, orientation_x,
             orientation_y, tp, flags, wavenumber, beam_enu, norm_enu,
@@ -909,15 +997,7 @@ int station_beam_aa(int num_stations, int num_elements, const T* el_x,
             beam};
     cudaStream_t s = as_stream(stream);
 #define OSKB_BEAM(D, NT)                                                     \
-    {                                                                        \
-        auto k = station_beam_kernel<T, D, NT, dirs_big<T>(NT),              \
-                kDirsSmall<T>>;                                              \
-        const int smem = (int) sizeof(BeamSmem<T, D, NT>);                   \
-        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                smem);                                                       \
-        k<<<grid, threads, smem, s>>>(arg, blocks, full, parts, first,       \
-                (unsigned) total);                                           \
-    }
+    launch_beam<T, D, NT>(arg, split, s);
 #define OSKB_BEAM_NT(D)                                                      \
     switch (num_element_types)                                               \
     {                                                                        \

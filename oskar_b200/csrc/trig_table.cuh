@@ -108,7 +108,9 @@ __device__ __forceinline__ void trig_steps_checked(const double2* table,
 // ---------------------------------------------------------------------------
 // The station beam's larger tables, with shorter series. Entry j of copy c is
 // element kCopies j + c, as above (FP32: 16 copies of 8-byte entries, for
-// half-warp requests). N entries: h = 2 pi / N, |x| = |h f| <= pi / N.
+// half-warp requests). N entries: h = 2 pi / N, |x| = |h f| <= pi / N. The
+// fill takes the first quadrant's entries from the library and turns them, so
+// that a small CTA has two sines to form instead of eight.
 //   FP64, N = 512 (64 KB): sin to x^5 (the omitted x^7/7! < 7e-20) and
 //     cos - 1 to x^4 with the x^6 term economised into the lower two
 //     (Chebyshev; what is left is below 5e-18): 13 operations.
@@ -117,6 +119,43 @@ __device__ __forceinline__ void trig_steps_checked(const double2* table,
 // The caller bounds the phase: |u| < kLimit, where round(u) still sits in
 // the low bits of u + 1.5 x 2^52 (FP32: 2^23).
 // ---------------------------------------------------------------------------
+__device__ __forceinline__ void sincos_half_turns(double x, double* s,
+        double* c)
+{
+    sincospi(x, s, c);
+}
+__device__ __forceinline__ void sincos_half_turns(float x, float* s, float* c)
+{
+    sincospif(x, s, c);
+}
+
+// Fills COPIES copies of the N entries (cos, sin)(2 pi j / N) from those of
+// the first quadrant: every thread takes one entry of it at a time and writes
+// it turned by 0, 1, 2 and 3 right angles; where the CTA has more threads
+// than the quadrant entries, several threads share an entry's four turns.
+template <int N, int COPIES, typename T2>
+__device__ __forceinline__ void trig_fill_quadrants(T2* table)
+{
+    constexpr int Q = N / 4;
+    const int share = min(4, max(1, (int) blockDim.x / Q));  // 1, 2 or 4
+    for (int i = threadIdx.x; i < Q * share; i += blockDim.x)
+    {
+        const int j = i % Q;
+        T2 e;   // (cos, sin)
+        sincos_half_turns((decltype(e.x)) j / (N / 2), &e.y, &e.x);
+        for (int q = i / Q; q < 4; q += share)
+        {
+            T2 v = e;
+            if (q & 1) { v.x = 0 - e.y; v.y = e.x; }
+            if (q & 2) { v.x = 0 - v.x; v.y = 0 - v.y; }
+            // (each lane starts at its own copy: distinct banks)
+#pragma unroll
+            for (int k = 0; k < COPIES; ++k)
+                table[(j + q * Q) * COPIES + ((k + j) & (COPIES - 1))] = v;
+        }
+    }
+}
+
 template <typename T> struct Trig;
 
 template <> struct Trig<double>
@@ -129,16 +168,7 @@ template <> struct Trig<double>
 
     static __device__ __forceinline__ void fill(Entry* table)
     {
-        for (int j = threadIdx.x; j < kEntries; j += blockDim.x)
-        {
-            double s, c;
-            sincospi((double) j / (kEntries / 2), &s, &c);
-            // (each lane starts at its own copy: distinct banks)
-#pragma unroll
-            for (int k = 0; k < kCopies; ++k)
-                table[j * kCopies + ((k + j) & (kCopies - 1))] =
-                        make_double2(c, s);
-        }
+        trig_fill_quadrants<kEntries, kCopies>(table);
     }
     static __device__ __forceinline__ void sincos(const Entry* table,
             double u, double* s, double* c)
@@ -181,29 +211,42 @@ template <> struct Trig<float>
     static constexpr int kSize = kEntries * kCopies;
     static constexpr double kStepsPerRadian = 40.74366543152521;  // 128 / pi
     static constexpr float kLimit = 2097152.0f;
+    static constexpr float kShift = 12582912.0f;  // 1.5 x 2^23
+    static constexpr double h = 3.141592653589793 / (kEntries / 2);
+    static constexpr float s1 = (float) h, s3 = (float) (-h * h * h / 6.0);
+    // f2^2 on [0, 1/4] as f2 / 4 (- 1/128)
+    static constexpr float c2 = (float) (-h * h / 2.0 + h * h * h * h / 24.0
+            / 4.0);
+
+    // The entry of round(u), in the low bits of t = u + kShift, turned by
+    // the remainder's sine and cosine - 1.
+    static __device__ __forceinline__ void rotate(const Entry* table, float t,
+            float sr, float cm, float* s, float* c)
+    {
+        const int n = __float_as_int(t);
+        const Entry e = table[((n & (kEntries - 1)) * kCopies) |
+                (threadIdx.x & (kCopies - 1))];
+        *c = fmaf(e.x, cm, fmaf(-e.y, sr, e.x));
+        *s = fmaf(e.y, cm, fmaf(e.x, sr, e.y));
+    }
 
     static __device__ __forceinline__ void fill(Entry* table)
     {
-        for (int j = threadIdx.x; j < kEntries; j += blockDim.x)
-        {
-            float s, c;
-            sincospif((float) j / (kEntries / 2), &s, &c);
-#pragma unroll
-            for (int k = 0; k < kCopies; ++k)
-                table[j * kCopies + ((k + j) & (kCopies - 1))] =
-                        make_float2(c, s);
-        }
+        trig_fill_quadrants<kEntries, kCopies>(table);
+    }
+    // One phase.
+    static __device__ __forceinline__ void sincos(const Entry* table, float u,
+            float* s, float* c)
+    {
+        const float t = u + kShift;
+        const float f = u - (t - kShift);
+        const float f2 = f * f;
+        rotate(table, t, f * fmaf(f2, s3, s1), f2 * c2, s, c);
     }
     // Two phases as a packed pair.
     static __device__ __forceinline__ void sincos2(const Entry* table,
             f32x2 u, float* s, float* c)
     {
-        constexpr float kShift = 12582912.0f;  // 1.5 x 2^23
-        constexpr double h = 3.141592653589793 / (kEntries / 2);
-        constexpr float s1 = (float) h, s3 = (float) (-h * h * h / 6.0);
-        // f2^2 on [0, 1/4] as f2 / 4 (- 1/128)
-        constexpr float c2 = (float) (-h * h / 2.0 + h * h * h * h / 24.0 /
-                4.0);
         const f32x2 t = add2(u, pack2(kShift, kShift));
         const f32x2 f = fma2(add2(t, pack2(-kShift, -kShift)),
                 pack2(-1.0f, -1.0f), u);
@@ -216,13 +259,7 @@ template <> struct Trig<float>
         unpack2(cm2, cm[0], cm[1]);
 #pragma unroll
         for (int j = 0; j < 2; ++j)
-        {
-            const int n = __float_as_int(tt[j]);
-            const Entry e = table[((n & (kEntries - 1)) * kCopies) |
-                    (threadIdx.x & (kCopies - 1))];
-            c[j] = fmaf(e.x, cm[j], fmaf(-e.y, sr[j], e.x));
-            s[j] = fmaf(e.y, cm[j], fmaf(e.x, sr[j], e.y));
-        }
+            rotate(table, tt[j], sr[j], cm[j], &s[j], &c[j]);
     }
     static __device__ __forceinline__ void exact(float u, float* s, float* c)
     {
@@ -231,15 +268,8 @@ template <> struct Trig<float>
     static __device__ __forceinline__ void checked(const Entry* table,
             float u, float* s, float* c)
     {
-        if (!(fabsf(u) < kLimit))
-        {
-            exact(u, s, c);
-            return;
-        }
-        float s2[2], c2[2];
-        sincos2(table, pack2(u, u), s2, c2);
-        *s = s2[0];
-        *c = c2[0];
+        if (fabsf(u) < kLimit) sincos(table, u, s, c);
+        else exact(u, s, c);
     }
 };
 
