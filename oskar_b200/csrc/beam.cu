@@ -75,7 +75,7 @@ template <typename T>
 struct TypeParams
 {
     T kL[kMaxTypes];      // dipole length x pi f / c
-    T cos_kL[kMaxTypes];
+    T cos_kL[kMaxTypes], sin_kL[kMaxTypes];
     int kind[kMaxTypes];  // 0 dipole, 1 isotropic
     int taper[kMaxTypes]; // 0 none, 1 cos(theta)^p, 2 Gaussian in theta
     T taper_param[kMaxTypes];  // p, or 4 ln 2 / FWHM^2
@@ -114,7 +114,7 @@ __device__ __forceinline__ void direction_pattern(const TypeParams<T>& tp,
     }
     if constexpr (sizeof(T) == 8)
         element_pattern_rotated<T>(X, Y, Z, dphi1, dphi2, rot, tp.kL[t],
-                tp.cos_kL[t], swap_xy, p);
+                tp.cos_kL[t], tp.sin_kL[t], swap_xy, p);
     else
         element_pattern<T>(X, Y, Z, false, dphi1, dphi2, tp.kL[t],
                 tp.cos_kL[t], swap_xy, p);
@@ -833,6 +833,7 @@ int make_type_params(int num_types, const double* dipole_length_m,
                 dipole_length_m[t] * (kPi * frequency_hz / c0) : 0.0;
         tp->kL[t] = (T) kL;
         tp->cos_kL[t] = (T) cos(kL);
+        tp->sin_kL[t] = (T) sin(kL);
         tp->kind[t] = on && element_kind ? element_kind[t] : 0;
         tp->taper[t] = on && taper_kind ? taper_kind[t] : 0;
         if (tp->kind[t] < 0 || tp->kind[t] > 1 || tp->taper[t] < 0 ||

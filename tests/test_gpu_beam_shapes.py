@@ -110,6 +110,44 @@ def test_table_phase_factors(real, entries, steps, bound, reach, num_dir):
     assert np.all(got[:3, 0] == 1) and np.all(got[:3, 1] == 0)
 
 
+@pytest.mark.parametrize("length", [0.7, 1.36, 2.9])
+def test_pattern_towards_the_dipole_axis(length):
+    """FP64: one dipole at the origin along x (its pattern is the beam), from
+    across it down to 1e-7 rad from its axis, against long double. (cos(kL a)
+    - cos kL) / (1 - a^2) is formed there as 2 sin(kL (1 + a) / 2) sin(kL (1 -
+    a) / 2) / (1 - a^2) with 1 - a^2 = |(y, z)|^2 / |d|^2. The quotient's
+    parts are a few roundings each: 2e-15, of the larger of the value and the
+    two sines' product near the pattern's own zeros."""
+    freq = 110e6
+    rng = np.random.default_rng(8)
+    off = 10.0 ** np.linspace(-7, 0.19, 4000)
+    tilt = rng.uniform(0, 0.5 * np.pi, 4000)
+    d = [np.cos(off) * np.where(rng.random(4000) < 0.5, -1, 1),
+         np.sin(off) * np.cos(tilt) * np.where(rng.random(4000) < 0.5, -1, 1),
+         np.sin(off) * np.sin(tilt)]
+    z = torch.zeros(1, dtype=torch.float64, device="cuda")
+    out = torch.zeros((1, 4000, 8), dtype=torch.float64, device="cuda")
+    up = dev(np.array([[0.0, 0.0, 1.0]]))
+    ob.call("oskb_station_beam_aa_d", 1, 1, z, z, z, None, None, None, None,
+            z, z, length, 0, 0, 0, 0, 0, freq, up, up, 4000,
+            *[dev(c) for c in d], 0, out, ob.stream_ptr())
+    got = out.cpu().numpy()[0]
+    kl = np.longdouble(length * (np.pi * freq / C0))
+    x, y, w = (c.astype(np.longdouble) for c in d)
+    h2 = x * x + y * y + w * w
+    rho2 = x * x + y * y
+    one_a2 = (y * y + w * w) / h2
+    a = np.abs(x) / np.sqrt(h2)
+    num = 2 * np.sin(kl * (1 + a) / 2) * np.sin(kl * one_a2 / (1 + a) / 2)
+    theta = -x * w / np.sqrt(rho2 * h2) * num / one_a2
+    phi = y / np.sqrt(rho2) * num / one_a2
+    size = np.abs(2 * np.sin(kl * one_a2 / (1 + a) / 2) / one_a2)
+    for col, want, scale in ((0, theta, x * w / np.sqrt(rho2 * h2)),
+                             (2, phi, y / np.sqrt(rho2))):
+        bound = 4e-15 * np.abs(scale) * size
+        assert np.all(np.abs(got[:, col] - want) <= bound)
+
+
 def test_largest_direction_count():
     """2^31 - 1 directions: the last block reaches past the largest int. The
     same direction throughout, so every output is the first one; 26 GB."""
