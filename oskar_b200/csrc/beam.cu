@@ -402,7 +402,8 @@ __device__ __forceinline__ void station_beam_item(BeamSmem<T, IS3D, NT>& sm,
     // The station's terms, by lanes of the last warp, which has the fewest
     // elements to stage: beside the other warps' staging where the element
     // loop is short, else beside their loops (128 stations x 12,000
-    // directions FP64: 564 us against 576 before the staging).
+    // directions FP64: 564 us against 576 before the staging; the choice at
+    // run time, with both copies of the code, took 1 to 8 % longer).
     const int lane = threadIdx.x & 31;
     const int term = threadIdx.x >= threads - 32 && lane < 2 * NT ? lane : -1;
     for (int e0 = 0; e0 < num_elements; e0 += kChunk)
@@ -880,14 +881,13 @@ int beam_ctas_per_sm(int threads)
 // directions x 1 to 4 element types, both precisions, with every choice
 // timed: the choice is 0.5 % above the best on average. Against one direction
 // per thread on 128 threads and the 128-entry table (FP64) or sincosf (FP32)
-// calls of all sizes take 0.77 (FP64) and 0.63 (FP32) of the time; of 900
-// shapes 13 take 1 to 9 % more, and 18 stations x 17 elements x 9,053
-// directions FP32, whose time is the patterns', 24 %.
+// calls of all sizes take 0.78 (FP64) and 0.63 (FP32) of the time; of 900
+// shapes 22 take 1 to 9 % more, and 18 stations x 17 elements x 9,053
+// directions FP32, whose time is the patterns', 26 %.
 template <typename T>
 BeamSplit beam_split(int num_stations, int num_elements, int num_directions,
         int num_types)
 {
-    constexpr bool f64 = sizeof(T) == 8;
     const int sms = device_sm_count(), big = dirs_big<T>(num_types);
     const auto ceil_div = [](long long a, long long b)
     {
@@ -907,24 +907,32 @@ BeamSplit beam_split(int num_stations, int num_elements, int num_directions,
         for (int small = kDirsSmall<T>; small >= 1; small /= 2)
             for (int threads = kThreads; threads >= 64; threads /= 2)
             {
-                const double ctas = (double) ceil_div(ceil_div(num_directions,
-                        threads * small) * num_stations, sms);
-                const double rounds = ceil(ctas / beam_ctas_per_sm<T>(
-                        threads));
+                const double n = num_elements, total = (double) (ceil_div(
+                        num_directions, threads * small) * num_stations);
+                const int per_sm = beam_ctas_per_sm<T>(threads);
+                const double ctas = ceil(total / sms), rounds = ceil(ctas /
+                        per_sm), all = ctas * threads;
                 const double staging = (double) ceil_div(std::min(
-                        num_elements, kChunk), threads) * std::max(1.0,
-                        (double) num_elements / kChunk);
-                // (FP32: one direction at a time takes 1.3 times its share
-                // of a pair; FP64: warps without directions take less)
-                const double work = f64 ? 1.0 : small == 1 ? 1.3 : small;
-                const double all = ctas * threads, live = std::max<double>(
-                        threads, 32.0 * ceil_div(num_directions, 32 * small) *
-                        num_stations / sms);
-                const double cost = rounds * (small * ((f64 ? 0.08 : 0.4) *
-                        num_elements + (f64 ? 2.4 : 12.0) * num_types) +
-                        40.0 * staging) + (f64 ? 0.68 * all + 0.32 * live :
-                        all) * work / 256.0 * num_elements + (f64 ? 7.5 :
-                        10.0) * 256 / threads;
+                        num_elements, kChunk), threads) * std::max(1.0, n /
+                        kChunk);
+                double cost = rounds * 40.0 * staging;
+                if constexpr (sizeof(T) == 8)
+                {
+                    // warps without directions take less; a last warp with
+                    // elements stages them after the station's terms
+                    const double live = std::max<double>(threads, 32.0 *
+                            ceil_div(num_directions, 32) * num_stations / sms);
+                    cost += (0.68 * all + 0.3 * live) / 256.0 * n + 0.17 * n *
+                            std::max(1.0, total / (per_sm * sms)) + 4.0 *
+                            256 / threads;
+                    if (num_elements > threads - 32) cost += 12.0 * rounds;
+                }
+                else
+                    // (one direction at a time takes 1.3 times its share of
+                    // a pair)
+                    cost += rounds * small * (0.4 * n + 12.0 * num_types) +
+                            all * (small == 1 ? 1.3 : small) / 256.0 * n +
+                            10.0 * 256 / threads;
                 if (best == 0 || cost < best)
                 {
                     best = cost;
