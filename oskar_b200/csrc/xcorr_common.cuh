@@ -36,8 +36,7 @@ struct XcorrParams
     T* vis;
     // Items: num_times x num_channels x tiles x slices, in that nesting
     // (slices fastest). Source slice y covers [y * slice_len,
-    // (y + 1) * slice_len). With more than one slice (single call only),
-    // each CTA writes its sums to partial[y][baseline][comp] and
+    // (y + 1) * slice_len). With more than one slice each CTA writes its sums to partial[y][baseline][comp] and
     // reduce_partials adds them to vis in slice order (deterministic).
     int num_times, num_channels, tiles, slices, slice_len;
     int tile_major;  // item order: tile outermost instead of innermost
@@ -94,13 +93,6 @@ __device__ __forceinline__ void cp_async_commit()
 __device__ __forceinline__ void cp_async_wait_all()
 {
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-}
-
-// Waits until at most N of this thread's cp.async groups are pending.
-template <int N>
-__device__ __forceinline__ void cp_async_wait_group()
-{
-    asm volatile("cp.async.wait_group %0;\n" :: "n"(N) : "memory");
 }
 
 // Maps a linear block index to (bp, bq) with bp >= bq.

@@ -10,11 +10,12 @@
 //
 // One CTA of 512 threads owns a 32 x 32 station tile, its 16 warps an 8 x 8
 // station patch each, two baselines per thread (FP64: two rows p; FP32: two
-// columns q, as packed pairs). Two baselines keep a thread under 128
-// registers, so 16 warps fit an SM: with four baselines per thread 8 warps
-// of 248 registers were latency-bound (FP64 pipe 35 % active; now 58 %, and
-// what is left is the latency of a source's chain of loads, reciprocal and
-// select with four warps per scheduler). A warp whose patch holds no baseline
+// columns q, as packed pairs). Two baselines keep a thread within 128
+// registers (most FP64 matrix forms at 128, spilling up to 24 bytes), so 16
+// warps fit an SM: with four baselines per thread 8 warps of 248 registers
+// were latency-bound (FP64 pipe 35 % active; now 58 %, and what is left is
+// the latency of a source's chain of loads, reciprocal and select with four
+// warps per scheduler). A warp whose patch holds no baseline
 // (above the diagonal, past the last station) skips the arithmetic; the
 // patches are dealt so that a diagonal tile's ten live ones spread over the
 // four schedulers.
@@ -28,9 +29,9 @@
 // serial transform of some overlaps the products of the others.
 //
 // Measured on one B200, 30 % Gaussian sources, both smearings, against the
-// four-baseline kernel: 256 stations x 20,000 sources x 4 channels FP64 19.8
-// ms (30.5 before: 132 G source-baselines/s against 86); 211 stations x
-// 9,001 sources x 6 FP32 6.5 ms (9.4).
+// four-baseline kernel: 256 stations x 20,000 sources x 4 channels FP64 20.1
+// ms (30.5 before: 130 G source-baselines/s against 86); 211 stations x
+// 9,001 sources x 6 FP32 5.8 ms (9.5).
 #pragma once
 
 #include "f32x2.cuh"
@@ -100,9 +101,10 @@ struct SmearSmem
 // |d| = tau the series of sinc is summed instead. FP64, tau = 1/16: 1 - y/6 +
 // y^2/120 - y^3/5040 + y^4/362880 (y = d^2; the next term is below 3e-20)
 // with the y^4 term economised into the lower ones (Chebyshev on [0, tau^2]:
-// y^4 = 2 t y^3 - 5/4 t^2 y^2 + 1/4 t^3 y to within t^4/128, t = tau^2; the
-// remainder is below 6e-18). FP32, tau = 1/2: the five terms (next: 3e-11).
-// Above tau the identity's relative error is below ~1e-14 (FP64) and ~1e-6
+// y^4 = 2 t y^3 - 5/4 t^2 y^2 + 1/4 t^3 y to within t^4/64, t = tau^2, the
+// constant t^4/128 left out as well; the remainder is 1.0e-17). FP32, tau =
+// 1/2: the five terms (next: 3e-11). Above tau the identity's relative error
+// is below ~1e-14 (FP64; measured 3.4e-15 from 0 to 700 rad) and ~1e-6
 // (FP32). Both forms are evaluated and one selected (no divergence within a
 // warp), as a numerator and a denominator (sin d, d) or (series, 1), so that
 // the bandwidth and time factors of a source-baseline share one reciprocal.
@@ -140,10 +142,11 @@ __device__ __forceinline__ void sinc_parts(double d, double by_identity,
 }
 
 // num / den for |den| >= 1/256: the hardware's reciprocal approximation y
-// (relative error e = 1 - den y below 2^-22), and the quotient num y
-// corrected by 1 / (1 - e) = 1 + e + e^2 (+ e^3 < 2^-66): a short dependent
-// chain instead of the IEEE division's; within an ulp or two of the
-// correctly rounded quotient.
+// (20 bits of den give 20 bits: e = 1 - den y is at most about 2^-19), and
+// the quotient num y corrected by 1 / (1 - e) = 1 + e + e^2 (+ e^3 < 2^-57):
+// a short dependent chain instead of the IEEE division's; within an ulp or
+// two of the correctly rounded quotient (a whole call's error is that with
+// the division to three digits).
 __device__ __forceinline__ double quotient(double num, double den)
 {
     double y;
@@ -218,18 +221,15 @@ __device__ __forceinline__ float max_or_nan(float a, float b)
     return __uint_as_float(max(__float_as_uint(a), __float_as_uint(b)));
 }
 
-// Whether every phase difference of a chunk is below tau: reach is the
+// FP32: whether every phase difference of a chunk is below tau: reach is the
 // chunk's largest |(l, m, n - 1)|, bw and ts the longest baseline in phase
-// units (0 without that smearing). False for NaN. The series alone is taken
-// in FP32 only, where tau = 1/2 covers arrays of a few km (125 stations x
-// 7,000 sources, 3 km: 2.6 times the four-baseline kernel, 1.6 without); in
-// FP64 tau = 1/16 seldom holds, and the second loop cost 3 to 5 % where it
-// did not.
-template <typename T>
+// units (0 without that smearing). False for NaN. The series alone is then
+// taken, as in arrays of a few km (211 stations x 9,001 sources x 6, 2 km:
+// 6.2 -> 5.8 ms); in FP64 tau = 1/16 seldom holds, and a second loop cost 3
+// to 5 % where it did not.
 __device__ __forceinline__ bool sinc_small(float reach, float bw, float ts)
 {
-    return sizeof(T) == 4 && reach * bw < (float) kSincTau<T> &&
-            reach * ts < (float) kSincTau<T>;
+    return reach * bw < kSincTau<float> && reach * ts < kSincTau<float>;
 }
 
 // Stores one element's factor values.
@@ -263,10 +263,9 @@ __device__ __forceinline__ void put_entry(SmearFactors<float, NC>& f,
 // 600 with the rounded steps).
 template <int NC>
 __device__ __forceinline__ void put_phase(SmearFactors<double, NC>& f,
-        int which, int blk, int sl, int stl, double ph, bool small)
+        int which, int blk, int sl, int stl, double ph, bool)
 {
     f.phi[which][blk][sl][stl] = ph;
-    if (small) return;
     double sn, cs;
     sincos(ph, &sn, &cs);
     f.sc[which][blk][sl][stl] = make_double2(sn, cs);
@@ -411,8 +410,8 @@ __device__ __forceinline__ void smear_transform(SmearSmem<T, MATRIX>& sm,
             reach = __uint_as_float(__reduce_max_sync(0xffffffffu,
                     __float_as_uint(r)));
         }
-        const bool small = sinc_small<T>(reach, __uint_as_float(sm.bound[0]),
-                __uint_as_float(sm.bound[1]));
+        const bool small = sizeof(T) == 4 && sinc_small(reach,
+                __uint_as_float(sm.bound[0]), __uint_as_float(sm.bound[1]));
         if (BW)
             put_phase(f, 0, blk, sl, stl, (T) (((double) u[0] * l +
                     (double) u[1] * m + (double) u[2] * n1) * prm.bw_scale),
@@ -426,8 +425,7 @@ __device__ __forceinline__ void smear_transform(SmearSmem<T, MATRIX>& sm,
 }
 
 // One chunk's products, FP64: the thread's rows pr, pr + 1 and column qc.
-// SMALL: every phase difference of the warp's patch is below tau.
-template <bool MATRIX, bool GAUSS, bool BW, bool TS, bool CASA, bool SMALL>
+template <bool MATRIX, bool GAUSS, bool BW, bool TS, bool CASA>
 __device__ __forceinline__ void smear_products(
         const SmearFactors<double, MATRIX ? 4 : 1>& f, int ns, int pr, int qc,
         const double (&uu2)[2], const double (&vv2)[2],
@@ -439,22 +437,7 @@ __device__ __forceinline__ void smear_products(
     {
         // ---- factors of the two baselines
         double w[2] = {1.0, 1.0};
-        if ((BW || TS) && SMALL)
-        {
-#pragma unroll
-            for (int which = BW ? 0 : 1; which < (TS ? 2 : 1); ++which)
-            {
-                const double pb = f.phi[which][1][sl][qc];
-#pragma unroll
-                for (int i = 0; i < 2; ++i)
-                {
-                    const double x = sinc_series(
-                            f.phi[which][0][sl][pr + i] - pb);
-                    w[i] = BW && which == 1 ? w[i] * x : x;
-                }
-            }
-        }
-        else if (BW || TS)
+        if (BW || TS)
         {
             double num[2], den[2];
 #pragma unroll
@@ -526,6 +509,7 @@ __device__ __forceinline__ void smear_products(
 
 // One chunk's products, FP32: the thread's row pr and columns qc, qc + 1 as
 // packed pairs; the chunk's sums are added to the FP64 sums at its end.
+// SMALL: every phase difference of the warp's patch is below tau.
 template <bool MATRIX, bool GAUSS, bool BW, bool TS, bool CASA, bool SMALL>
 __device__ __forceinline__ void smear_products(
         const SmearFactors<float, MATRIX ? 4 : 1>& f, int ns, int pr, int qc,
@@ -835,7 +819,10 @@ xcorr_smear_kernel(const XcorrParams<T> prm)
             }
             else if (active)
             {
-                if ((BW || TS) && sinc_small<T>(reach, longest[0],
+                if constexpr (F64)
+                    smear_products<MATRIX, GAUSS, BW, TS, CASA>(sm.f[c & 1],
+                            ns, pr, qc, uu2, vv2, uuvv, acc);
+                else if ((BW || TS) && sinc_small(reach, longest[0],
                         longest[1]))
                     smear_products<MATRIX, GAUSS, BW, TS, CASA, true>(
                             sm.f[c & 1], ns, pr, qc, uu2, vv2, uuvv, acc);

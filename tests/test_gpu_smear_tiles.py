@@ -42,10 +42,10 @@ def test_patches_chunks_and_mixed_sources(num_st, num_src, real, matrix, bw,
 @pytest.mark.parametrize("bw,ts", [(100e3, 0.0), (0.0, 10.0), (100e3, 10.0)])
 @pytest.mark.parametrize("core", [0, 8, 20, 70])
 def test_short_and_long_baselines(real, bw, ts, core):
-    """Patches whose phase differences are all small take the series alone,
-    the others the identity too: a core of stations within 60 m (FP64) or
-    400 m (FP32) and the rest up to 60 (6) km, from none of one to none of
-    the other. FP32 phases of 0.02 x 6 km carry 120 x 6e-8 absolute error:
+    """FP32 patches whose phase differences are all small take the series
+    alone, the others (and FP64) select it per baseline: a core of stations
+    within 60 m (FP64) or 400 m (FP32) and the rest up to 60 (6) km, from none
+    of one to none of the other. FP32 phases of 0.02 x 6 km carry 120 x 6e-8 absolute error:
     1e-5 as above."""
     c = XcorrCase(70, 57, real=real, ranges="physical", bandwidth_hz=bw,
                   time_avg=ts, gaussian=False, seed=core + 1)
